@@ -194,7 +194,8 @@ def run(state):
         n = _lib.finalize(state["res"].data_ptr(), state["val"].data_ptr(), plan.group_slots, plan.storage_ts,
                           state["types"], state["nullable"], plan.sparse, not plan.groups, list(plan.order_by),
                           state["limit"], state["cols"].data_ptr(), state["cval"].data_ptr(), state["cap"], _stream())
-        return n, state["cols"], state["cval"]
+        # The rows asked for (past the last row both buffers stay as they were).
+        return n, state["cols"].view(plan.visible_ts, -1)[:, :state["limit"]], state["cval"]
     _lib.check(state["fn"](state["res"].data_ptr(), plan.group_slots, plan.storage_ts, state["dst"].data_ptr(),
                            state["count"].data_ptr(), _stream()), "compaction")
     return state["dst"], state["count"]
