@@ -26,23 +26,71 @@ int invalid(const char* what) { return cx_internal::set_error(CX_E_INVALID, what
 constexpr int kCompactBlock = 256;
 constexpr int kCompactPerBlock = 2048;  // groups per block
 
-// Pass 1: number of present groups (any non-zero slot) per block of groups.
+constexpr unsigned long long kCompactSelfScan = 2048;  // most blocks whose write pass sums the counts itself
+
+// Presence flags of the block's groups [g0, g0 + n): the tuples are read as one
+// stream of words (two per load where the table is 16-byte aligned; g0 * ts is
+// even), and a non-zero word marks its group.  A thread per tuple read the same
+// bytes in loads of stride 8 * ts, ten lines each for five-word tuples.
+__device__ __forceinline__ void compact_flags(const unsigned long long* __restrict__ src, unsigned long long g0,
+                                              unsigned n, unsigned ts, unsigned char* s_flag) {
+  for (unsigned i = threadIdx.x; i < kCompactPerBlock / 4; i += kCompactBlock) ((unsigned*)s_flag)[i] = 0u;
+  __syncthreads();
+  const unsigned long long* base = src + g0 * ts;
+  const unsigned long long words = (unsigned long long)n * ts;
+  const bool narrow = ts <= (1u << 20);  // word numbers of a block fit 32 bits: no 64-bit division
+  auto group_of = [&](unsigned long long w) -> unsigned { return narrow ? (unsigned)w / ts : (unsigned)(w / ts); };
+  if ((((unsigned long long)src) & 15ULL) == 0ULL) {
+    const unsigned long long pairs = words / 2;
+    const ulonglong2* v = (const ulonglong2*)base;
+    unsigned long long i = threadIdx.x;
+    for (; i + 3 * kCompactBlock < pairs; i += 4 * kCompactBlock) {
+      ulonglong2 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = __ldcs(v + i + k * kCompactBlock);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const unsigned long long w = 2 * (i + k * kCompactBlock);
+        if (x[k].x) s_flag[group_of(w)] = 1;
+        if (x[k].y) s_flag[group_of(w + 1)] = 1;
+      }
+    }
+    for (; i < pairs; i += kCompactBlock) {
+      const ulonglong2 x = __ldcs(v + i);
+      if (x.x) s_flag[group_of(2 * i)] = 1;
+      if (x.y) s_flag[group_of(2 * i + 1)] = 1;
+    }
+    if ((words & 1) && threadIdx.x == 0 && base[words - 1]) s_flag[n - 1] = 1;
+  } else {
+    for (unsigned long long i = threadIdx.x; i < words; i += kCompactBlock)
+      if (base[i]) s_flag[group_of(i)] = 1;
+  }
+  __syncthreads();
+}
+
+// Pass 1: number of present groups (any non-zero slot) per block of groups and,
+// where `mask` has room, one presence bit per group, so that pass 3 reads the
+// present tuples and not the table again.
 __global__ void __launch_bounds__(kCompactBlock)
 compact_count(const unsigned long long* __restrict__ src, unsigned long long groups, unsigned ts,
-              unsigned long long* __restrict__ block_counts) {
+              unsigned long long* __restrict__ block_counts, unsigned* __restrict__ mask) {
+  __shared__ __align__(16) unsigned char s_flag[kCompactPerBlock];
+  __shared__ unsigned part[kCompactBlock / 32];
   const unsigned long long g0 = (unsigned long long)blockIdx.x * kCompactPerBlock;
-  unsigned long long cnt = 0;
-  for (unsigned long long g = g0 + threadIdx.x; g < g0 + kCompactPerBlock && g < groups; g += kCompactBlock) {
-    bool present = false;
-    for (unsigned c = 0; c < ts && !present; ++c) present = src[g * ts + c] != 0ULL;
-    cnt += present;
+  const unsigned n = (unsigned)(groups - g0 < kCompactPerBlock ? groups - g0 : kCompactPerBlock);
+  compact_flags(src, g0, n, ts, s_flag);
+  unsigned cnt = 0;
+  for (unsigned i = threadIdx.x; i < kCompactPerBlock; i += kCompactBlock) {
+    const unsigned m = __ballot_sync(0xffffffffu, s_flag[i]);
+    if ((threadIdx.x & 31) == 0) {
+      cnt += __popc(m);
+      if (mask) mask[(g0 + i) >> 5] = m;
+    }
   }
-  __shared__ unsigned long long part[kCompactBlock / 32];
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = cnt;
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned long long s = 0;
+    unsigned s = 0;
     for (int w = 0; w < kCompactBlock / 32; ++w) s += part[w];
     block_counts[blockIdx.x] = s;
   }
@@ -84,34 +132,68 @@ compact_scan(unsigned long long* counts, unsigned long long nblocks, unsigned lo
   if (threadIdx.x == 0) *total = carry;
 }
 
-// Pass 3: write present tuples in group order.
+// Pass 3: write present tuples in group order, as one stream of words per
+// block.  `offsets`: the blocks' exclusive prefix, or (total non-null) their
+// counts, which each block sums up to its own (at most 16 KB from L2, less than
+// the launch of a scan).  `mask` null: presence is read from the table again.
 __global__ void __launch_bounds__(kCompactBlock)
 compact_write(const unsigned long long* __restrict__ src, unsigned long long groups, unsigned ts,
-              const unsigned long long* __restrict__ offsets, unsigned long long* __restrict__ dst) {
+              const unsigned long long* __restrict__ offsets, const unsigned* __restrict__ mask,
+              unsigned long long* __restrict__ dst, unsigned long long* total) {
+  __shared__ __align__(16) unsigned char s_flag[kCompactPerBlock];
+  __shared__ unsigned short s_list[kCompactPerBlock];  // the block's present groups in order
+  __shared__ unsigned long long part[kCompactBlock / 32];
+  __shared__ unsigned s_before[kCompactPerBlock / 32 + 1];
   const unsigned long long g0 = (unsigned long long)blockIdx.x * kCompactPerBlock;
-  __shared__ unsigned long long warp_tot[kCompactBlock / 32];
-  __shared__ unsigned long long base_s;
-  if (threadIdx.x == 0) base_s = offsets[blockIdx.x];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (unsigned long long chunk = g0; chunk < g0 + kCompactPerBlock && chunk < groups; chunk += kCompactBlock) {
-    const unsigned long long g = chunk + threadIdx.x;
-    bool present = false;
-    if (g < groups && g < g0 + kCompactPerBlock)
-      for (unsigned c = 0; c < ts && !present; ++c) present = src[g * ts + c] != 0ULL;
-    const unsigned ballot = __ballot_sync(0xffffffffu, present);
-    if (lane == 0) warp_tot[warp] = __popc(ballot);
-    __syncthreads();
-    unsigned long long before = base_s;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    before += __popc(ballot & ((1u << lane) - 1u));
-    if (present)
-      for (unsigned c = 0; c < ts; ++c) dst[before * ts + c] = src[g * ts + c];
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 0; w < kCompactBlock / 32; ++w) base_s += warp_tot[w];
-    __syncthreads();
+  const unsigned n = (unsigned)(groups - g0 < kCompactPerBlock ? groups - g0 : kCompactPerBlock);
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long sum = 0;
+  if (total) {
+    for (unsigned b = threadIdx.x; b < blockIdx.x; b += kCompactBlock) sum += offsets[b];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
   }
+  if (lane == 0) part[warp] = sum;
+  if (!mask) compact_flags(src, g0, n, ts, s_flag);
+  constexpr unsigned kWords = kCompactPerBlock / 32;
+  for (unsigned w = warp; w < kWords; w += kCompactBlock / 32) {
+    const unsigned m = mask ? mask[(g0 >> 5) + w] : __ballot_sync(0xffffffffu, s_flag[w * 32 + lane]);
+    if (lane == 0) s_before[w + 1] = __popc(m);
+  }
+  __syncthreads();
+  unsigned long long before = total ? 0ULL : offsets[blockIdx.x];
+  if (total)
+    for (int w = 0; w < kCompactBlock / 32; ++w) before += part[w];
+  if (threadIdx.x == 0) {
+    s_before[0] = 0;
+    for (unsigned w = 1; w <= kWords; ++w) s_before[w] += s_before[w - 1];
+    if (total && blockIdx.x == gridDim.x - 1) *total = before + s_before[kWords];
+  }
+  __syncthreads();
+  for (unsigned w = warp; w < kWords; w += kCompactBlock / 32) {
+    const unsigned m = mask ? mask[(g0 >> 5) + w] : __ballot_sync(0xffffffffu, s_flag[w * 32 + lane]);
+    if ((m >> lane) & 1u) s_list[s_before[w] + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(w * 32 + lane);
+  }
+  __syncthreads();
+  const unsigned long long words = (unsigned long long)s_before[kWords] * ts;
+  for (unsigned long long i = threadIdx.x; i < words; i += kCompactBlock) {
+    const unsigned r = ts <= (1u << 20) ? (unsigned)i / ts : (unsigned)(i / ts);
+    dst[before * ts + i] = src[(g0 + s_list[r]) * ts + (i - (unsigned long long)r * ts)];
+  }
+}
+
+// The three passes with `counts` (a word per block) and, if not null, `mask`
+// (kCompactPerBlock bits per block) as scratch.  Measured on 8.25M five-word
+// groups with some 40,000 present (330 MB): 86 us with the mask, of which the one
+// read of the table takes 51 us at the copy peak; 129 us as a thread per tuple
+// reading the table twice.
+void compact_launch(const uint64_t* src, uint64_t groups, uint32_t ts, uint64_t* dst, uint64_t* dev_count,
+                    unsigned long long* counts, unsigned* mask, unsigned long long nblocks, cudaStream_t s) {
+  const bool self_scan = nblocks <= kCompactSelfScan;
+  unsigned long long* total = (unsigned long long*)dev_count;
+  compact_count<<<(unsigned)nblocks, kCompactBlock, 0, s>>>((const unsigned long long*)src, groups, ts, counts, mask);
+  if (!self_scan) compact_scan<<<1, 1024, 0, s>>>(counts, nblocks, total);
+  compact_write<<<(unsigned)nblocks, kCompactBlock, 0, s>>>((const unsigned long long*)src, groups, ts, counts, mask,
+                                                            (unsigned long long*)dst, self_scan ? total : nullptr);
 }
 
 __global__ void gen_uniform_kernel(unsigned long long stream, unsigned long long seed, long long lo, unsigned long long span,
@@ -167,12 +249,9 @@ extern "C" int cx_compact_sparse(const uint64_t* src, uint64_t groups, uint32_t 
     return e == cudaSuccess ? CX_OK : cuda_fail(e, "cudaMemsetAsync");
   }
   unsigned long long* counts = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&counts, nblocks * 8, s);
+  cudaError_t e = cudaMallocAsync((void**)&counts, nblocks * (8 + kCompactPerBlock / 8), s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync");
-  compact_count<<<(unsigned)nblocks, kCompactBlock, 0, s>>>((const unsigned long long*)src, groups, ts, counts);
-  compact_scan<<<1, 1024, 0, s>>>(counts, nblocks, (unsigned long long*)dev_count);
-  compact_write<<<(unsigned)nblocks, kCompactBlock, 0, s>>>((const unsigned long long*)src, groups, ts, counts,
-                                                            (unsigned long long*)dst);
+  compact_launch(src, groups, ts, dst, dev_count, counts, (unsigned*)(counts + nblocks), nblocks, s);
   e = cudaGetLastError();
   cudaFreeAsync(counts, s);
   return e == cudaSuccess ? CX_OK : cuda_fail(e, "compaction launch");
@@ -239,11 +318,9 @@ extern "C" int cx_compact_sparse_noalloc(const uint64_t* src, uint64_t groups, u
     counts = g_noalloc_ptr[dev];
   }
   // compact_count writes every one of the nblocks counts, so the array needs
-  // no clearing between calls.
-  compact_count<<<(unsigned)nblocks, kCompactBlock, 0, s>>>((const unsigned long long*)src, groups, ts, counts);
-  compact_scan<<<1, 1024, 0, s>>>(counts, nblocks, (unsigned long long*)dev_count);
-  compact_write<<<(unsigned)nblocks, kCompactBlock, 0, s>>>((const unsigned long long*)src, groups, ts, counts,
-                                                            (unsigned long long*)dst);
+  // no clearing between calls.  It has no room for presence bits (4 MiB at the
+  // maximum), so the write pass reads the table a second time.
+  compact_launch(src, groups, ts, dst, dev_count, counts, nullptr, nblocks, s);
   e = cudaGetLastError();
   return e == cudaSuccess ? CX_OK : cuda_fail(e, "compaction launch");
 }
