@@ -820,6 +820,50 @@ CX_DEVICE void raise(unsigned int* err, unsigned int code) {
   if (err) atomicCAS(err, 0u, code);
 }
 
+// Group tables of 32-bit shared-memory words (native atomics).
+// x into a (low, high) pair: the low word's carry goes into the high one, so
+// the pair is the sum modulo 2^64 in any order of adds.
+CX_DEVICE void add_lohi(unsigned* lo, unsigned* hi, unsigned long long x) {
+  const unsigned xl = (unsigned)x;
+  const unsigned old = atomicAdd(lo, xl);
+  const unsigned h = (unsigned)(x >> 32) + (old + xl < xl ? 1u : 0u);
+  if (h) atomicAdd(hi, h);
+}
+CX_DEVICE unsigned long long lohi(unsigned lo, unsigned hi) { return ((unsigned long long)hi << 32) | lo; }
+// Tested before the atomic: a word that another lane has changed since costs
+// one atomic that changes nothing.
+CX_DEVICE void set_bit_once(unsigned* word, unsigned bit) {
+  if (!(*word & bit)) atomicOr(word, bit);
+}
+CX_DEVICE void min_word(unsigned* word, unsigned x) {
+  if (x < *word) atomicMin(word, x);
+}
+CX_DEVICE void max_word(unsigned* word, unsigned x) {
+  if (x > *word) atomicMax(word, x);
+}
+// Over all 32 lanes, result in every lane.
+CX_DEVICE unsigned long long warp_sum_u64(unsigned long long x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+CX_DEVICE unsigned long long warp_min_u64(unsigned long long x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long y = __shfl_xor_sync(0xffffffffu, x, o);
+    x = y < x ? y : x;
+  }
+  return x;
+}
+CX_DEVICE unsigned long long warp_max_u64(unsigned long long x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long y = __shfl_xor_sync(0xffffffffu, x, o);
+    x = y > x ? y : x;
+  }
+  return x;
+}
+
 CX_DEVICE unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 CX_DEVICE void mbar_init(unsigned long long* bar, unsigned count) {

@@ -782,14 +782,53 @@ struct Emitter {
       lacc_off = (off + 15) & ~15ULL;
       off = lacc_off + G * NACC * 8ULL * CTA;
     }
+    // Shared-memory group tables of 32-bit words: a SUM is a low and a high word
+    // (the carry of the low add goes into the high one), a COUNT one word (two
+    // where a multi-value join can repeat a row without bound), MIN / MAX of an
+    // int32 column one word (sign extension keeps the unsigned order).  32-bit
+    // shared atomics are native; 64-bit ones are compare-and-swap loops, and
+    // merging equal groups across the warp first (__match_any_sync, then a
+    // shuffle per peer) costs more than the atomics it saves.  LREP copies of a
+    // word lie side by side, one per lane modulo LREP, so that 32 lanes on one
+    // group still hit 32 banks; as many copies as fit into the bytes that one
+    // 64-bit table per warp took (domains up to 256 groups), else one.
+    // Measured (60M rows, scan): OR-join with COUNT / MIN / MAX / AVG into 12
+    // groups 1.648 -> 0.427 ms (with or_probes below), multi-value join into 35
+    // groups 1.24 -> 0.87 ms, Q3.1 (4,375 groups) 0.224 -> 0.218 ms queued and
+    // 0.345 -> 0.306 ms unqueued, three joins into 175 groups 0.203 -> 0.195 ms.
+    // group_merge = 1 and MIN / MAX over expressions keep the 64-bit tables.
+    bool any_multi = false;
+    for (const auto& s : p.steps) any_multi = any_multi || (s.kind == Step::JoinStep && s.join.multi);
+    std::vector<int> w32_word(NA, 0);  // first word of each aggregate
+    int W32 = 0;
+    bool w32 = grouped && !reg_groups && !lane_groups && tu.group_merge != 1;
+    const int cnt_words = any_multi ? 2 : 1;
+    for (int k = 0; k < NA; ++k) {
+      const Agg& ag = p.aggs[k];
+      w32_word[k] = W32;
+      if (ag.fn == AggFn::Min || ag.fn == AggFn::Max) {
+        w32 = w32 && ag.arg->op == Op::Col;
+        W32 += 1;
+      } else {
+        W32 += (ag.fn == AggFn::Count ? 0 : 2) + (ag.fn == AggFn::Sum ? 0 : cnt_words);
+      }
+    }
+    int LREP = 1;
     if (grouped && !reg_groups && !lane_groups) {
       const unsigned long long one = G * NACC * 8 + TW * 4 * (1 + NSEEN_T);
       if (tu.group_placement == 1) smem_groups = true;
       else if (tu.group_placement == 2) smem_groups = false;
       else smem_groups = one <= (unsigned long long)tu.smem_group_budget;
+      w32 = w32 && smem_groups;
       if (smem_groups) {
         if (G <= 256 && one * NW <= (unsigned long long)tu.smem_group_budget) REP = NW;
-        acc_off = (off + 15) & ~15ULL; off = acc_off + (unsigned long long)REP * G * NACC * 8;
+        unsigned long long table = (unsigned long long)REP * G * NACC * 8;
+        if (w32) {
+          while (LREP < 32 && G * W32 * 4 * LREP * 2 <= table) LREP *= 2;
+          table = (G * W32 * 4 * LREP + 7) & ~7ULL;
+          REP = 1;
+        }
+        acc_off = (off + 15) & ~15ULL; off = acc_off + table;
         touch_off = off; off += (unsigned long long)REP * TW * 4;
         seen_off = off; off += (unsigned long long)REP * NSEEN_T * TW * 4;
       }
@@ -930,6 +969,18 @@ struct Emitter {
       o << "  unsigned rtouch = 0u;\n";
       for (int k = 0; k < NA; ++k)
         if (seen_idx[k] >= 0 && NSEEN_T > 0) o << "  unsigned rseen_" << k << " = 0u;\n";
+    } else if (w32) {
+      o << "  unsigned int* s_w32 = (unsigned int*)(cx_smem + " << acc_off << ");\n";
+      o << "  unsigned int* s_touch = (unsigned int*)(cx_smem + " << touch_off << "); (void)s_touch;\n";
+      o << "  unsigned int* s_seen = (unsigned int*)(cx_smem + " << seen_off << "); (void)s_seen;\n";
+      std::string min_words;
+      for (int k = 0; k < NA; ++k)
+        if (p.aggs[k].fn == AggFn::Min) min_words += (min_words.empty() ? "" : " || ") + std::string("s == ") + std::to_string(w32_word[k]);
+      o << "  for (unsigned w = threadIdx.x; w < " << G * W32 * LREP << "u; w += " << CTA << ") {\n";
+      if (!min_words.empty()) o << "    const unsigned s = w / " << LREP << "u % " << W32 << "u;\n";
+      o << "    s_w32[w] = " << (min_words.empty() ? "0u" : "(" + min_words + ") ? ~0u : 0u") << ";\n";
+      o << "  }\n";
+      o << "  for (unsigned w = threadIdx.x; w < " << TW * (1 + NSEEN_T) << "u; w += " << CTA << ") s_touch[w] = 0u;\n";
     } else if (smem_groups) {
       o << "  unsigned long long* s_acc_all = (unsigned long long*)(cx_smem + " << acc_off << ");\n";
       o << "  unsigned int* s_touch_all = (unsigned int*)(cx_smem + " << touch_off << ");\n";
@@ -1254,6 +1305,44 @@ struct Emitter {
           o << ii << "db::atomic_set_valid_bit(d_result_validity, " << row << " + " << slot << ");\n";
       }
     };
+    // 32-bit group tables: every active lane adds its own row.  Touched and
+    // seen bits are tested before they are set (an atomic only the first time),
+    // and MIN / MAX before they are lowered / raised; a stale read costs an
+    // atomic that changes nothing.  A COUNT(*) stands in for the touched bit.
+    const int star_slot = count_star_slot();
+    auto w32_update = [&](const std::string& ii) {
+      auto set_bit = [&](const std::string& words) {
+        o << ii << "cx::set_bit_once(&" << words << ", 1u << (hash & 31));\n";
+      };
+      o << ii << "unsigned* w_ = s_w32 + (unsigned)hash * " << W32 * LREP << "u"
+        << (LREP > 1 ? " + (lane & " + std::to_string(LREP - 1) + ")" : std::string()) << ";\n";
+      if (star_slot < 0) set_bit("s_touch[hash >> 5]");
+      for (int k = 0; k < NA; ++k) {
+        const Agg& ag = p.aggs[k];
+        const std::string v = ag.arg->op == Op::Star ? "1" : valid_of(ag.arg.get());
+        auto word = [&](int w) { return "&w_[" + std::to_string(w * LREP) + "]"; };
+        const int w0 = w32_word[k];
+        auto count = [&](int w) {
+          if (cnt_words == 1) o << ii << "  atomicAdd(" << word(w) << ", 1u);\n";
+          else o << ii << "  cx::add_lohi(" << word(w) << ", " << word(w + 1) << ", 1ULL);\n";
+        };
+        o << ii << "if (" << v << ") {\n";
+        switch (ag.fn) {
+          case AggFn::Count: count(w0); break;
+          case AggFn::Min: o << ii << "  cx::min_word(" << word(w0) << ", (unsigned)" << math_push(ag.arg.get(), false) << ");\n"; break;
+          case AggFn::Max: o << ii << "  cx::max_word(" << word(w0) << ", (unsigned)" << math_push(ag.arg.get(), false) << ");\n"; break;
+          default:
+            o << ii << "  cx::add_lohi(" << word(w0) << ", " << word(w0 + 1) << ", (unsigned long long)("
+              << math_push(ag.arg.get(), true) << "));\n";
+            if (ag.fn == AggFn::Avg) count(w0 + 2);
+        }
+        if (seen_idx[k] >= 0 && NSEEN_T > 0) {
+          o << ii << "  ";
+          o << "cx::set_bit_once(&s_seen[" << (unsigned long long)seen_idx[k] * TW << "u + (hash >> 5)], 1u << (hash & 31));\n";
+        }
+        o << ii << "}\n";
+      }
+    };
     auto item_consume = [&](const std::string& ii) {
       if (!grouped) return scalar_update(ii);
       o << ii << "{\n";
@@ -1261,6 +1350,7 @@ struct Emitter {
       o << ii << "  if ((unsigned)hash < " << G << "u) {\n";
       if (reg_groups) reg_update(ii + "    ");
       else if (lane_groups) lane_update(ii + "    ");
+      else if (w32) w32_update(ii + "    ");
       else atomic_update(ii + "    ");
       o << ii << "  }\n" << ii << "}\n";
     };
@@ -1279,6 +1369,19 @@ struct Emitter {
       }
       const Join& j = s.join;
       const std::string K = std::to_string(k), ht = ht_name(j.dim);
+      if (k == xs && !j.multi) {
+        // The OR-join's probes are done (or_probes): each branch is a hit bit.
+        for (size_t f = 0; f < j.fks.size(); ++f) {
+          const std::string F = std::to_string(f);
+          o << ii << "if ((or_hit_ >> (i * " << j.fks.size() << " + " << F << ")) & 1u) {\n";
+          if (!j.payload.empty()) o << ii << "  " << j.payload << "[i] = or_pay" << F << "_[i];\n";
+          if (!j.payload.empty() && payload_valid.count(j.payload))
+            o << ii << "  " << j.payload << "_valid[i] = (int)((or_val" << F << "_ >> i) & 1u);\n";
+          item_steps(k + 1, ii + "  ");
+          o << ii << "}\n";
+        }
+        return;
+      }
       for (size_t f = 0; f < j.fks.size(); ++f) {
         const std::string& fk = j.fks[f];
         std::vector<std::string> terms{valid_regs.count(fk) ? fk + "_valid[i]" : "1"};
@@ -1518,11 +1621,51 @@ struct Emitter {
       o << ii << "}\n";
     };
 
+    // Every probe of a leading OR-join before any expanded row is consumed: the
+    // loads of all items and fact keys are in flight together (key and payload
+    // of a slot in one 8-byte load), instead of one dependent pair per branch.
+    auto or_probes = [&](const std::string& ii) {
+      const Join& j = p.steps[xs].join;
+      const std::string ht = ht_name(j.dim);
+      const size_t F = j.fks.size();
+      const bool pay = !j.payload.empty(), pv_pay = pay && payload_valid.count(j.payload);
+      o << ii << (IPT * F > 32 ? "unsigned long long" : "unsigned") << " or_hit_ = 0u;\n";
+      for (size_t f = 0; f < F; ++f) {
+        if (pay) o << ii << "int or_pay" << f << "_[ITEMS_PER_THREAD];\n";
+        if (pv_pay) o << ii << "unsigned or_val" << f << "_ = 0u;\n";
+      }
+      for (size_t f = 0; f < F; ++f) {
+        const std::string& fk = j.fks[f];
+        std::vector<std::string> terms{"flags[i]", "(tid + BLOCK_THREADS * i < num_tile_items)", valid_regs.count(fk) ? fk + "_valid[i]" : "1"};
+        for (size_t q = 0; q < f; ++q) {
+          const std::string& pf = j.fks[q];
+          const std::string pv = valid_regs.count(pf) ? pf + "_valid[i]" : "1";
+          terms.push_back(lit_true(pv) ? fk + "[i] != " + pf + "[i]" : "(!(" + pv + ") || " + fk + "[i] != " + pf + "[i])");
+        }
+        o << ii << "#pragma unroll\n" << ii << "for (int i = 0; i < ITEMS_PER_THREAD; ++i) {\n";
+        o << ii << "  const int h_ = (" << and_terms(terms) << ") ? cx_detail::pht_slot<int>(" << fk << "[i], " << j.len << ", " << j.keymin
+          << ") : -1;\n";
+        if (pay) {
+          o << ii << "  int2 kv_ = make_int2(0, 0);\n";
+          o << ii << "  if (h_ >= 0) kv_ = ((const int2*)" << ht << ")[h_];\n";
+          o << ii << "  or_pay" << f << "_[i] = kv_.y;\n";
+        } else {
+          o << ii << "  int2 kv_ = make_int2(0, 0);\n";
+          o << ii << "  if (h_ >= 0) kv_.x = " << ht << "[h_];\n";
+        }
+        o << ii << "  const bool hit_ = h_ >= 0 && kv_.x == " << fk << "[i];\n";
+        o << ii << "  or_hit_ |= (" << (IPT * F > 32 ? "unsigned long long" : "unsigned") << ")hit_ << (i * " << F << " + " << f << ");\n";
+        if (pv_pay)
+          o << ii << "  if (hit_) or_val" << f << "_ |= ((" << ht << "_valid[h_ >> 5] >> (h_ & 31)) & 1u) << i;\n";
+        o << ii << "}\n";
+      }
+    };
     // Aggregate consume.
     auto emit_consume = [&](const std::string& ind) {
       if (uniform_expand) {
         uniform_expansion(ind);
       } else if (expanding) {
+        if (!p.steps[xs].join.multi) or_probes(ind);
         o << ind << "#pragma unroll\n" << ind << "for (int i = 0; i < ITEMS_PER_THREAD; ++i) {\n";
         o << ind << "  if (flags[i] && (tid + BLOCK_THREADS * i < num_tile_items)) {\n";
         item_steps(xs, ind + "    ");
@@ -1532,12 +1675,13 @@ struct Emitter {
         o << ind << "  if (flags[i] && (tid + BLOCK_THREADS * i < num_tile_items)) {\n";
         scalar_update(ind + "    ");
         o << ind << "  }\n" << ind << "}\n";
-      } else if (reg_groups || lane_groups) {
+      } else if (reg_groups || lane_groups || w32) {
         o << ind << "#pragma unroll\n" << ind << "for (int i = 0; i < ITEMS_PER_THREAD; ++i) {\n";
         o << ind << "  if (flags[i] && (tid + BLOCK_THREADS * i < num_tile_items)) {\n";
         group_hash(ind + "    ");
         o << ind << "    if ((unsigned)hash < " << G << "u) {\n";
         if (reg_groups) reg_update(ind + "      ");
+        else if (w32) w32_update(ind + "      ");
         else lane_update(ind + "      ");
         o << ind << "    }\n";
         o << ind << "  }\n";
@@ -1700,6 +1844,69 @@ struct Emitter {
           o << "      if (v_[" << avg_idx[k] << "] != 0ULL) atomicAdd(&d_result[(unsigned long long)g * " << TS << "ULL + " << p.hidden_count_slot(k) << "], v_[" << avg_idx[k] << "]);\n";
       }
       o << "    }\n";
+      o << "  }\n";
+    } else if (w32) {
+      // A warp per group where each lane has its own copy, else a thread.
+      const bool by_warp = LREP == 32;
+      o << "  __syncthreads();\n";
+      if (by_warp) o << "  for (int g = warp; g < " << G << "; g += NWARP) {\n";
+      else o << "  for (int g = threadIdx.x; g < " << G << "; g += " << CTA << ") {\n";
+      if (star_slot < 0) o << "    if (!((s_touch[g >> 5] >> (g & 31)) & 1u)) continue;\n";
+      o << "    const unsigned* w_ = s_w32 + (unsigned)g * " << W32 * LREP << "u" << (by_warp ? " + lane" : "") << ";\n";
+      for (int k = 0; k < NA; ++k) {
+        const Agg& ag = p.aggs[k];
+        const AggFn f = ag.fn;
+        auto reduce = [&](const std::string& var, const std::string& init, const std::string& fold, const std::string& warp_fn,
+                          const std::function<std::string(const std::string&)>& value) {
+          o << "    unsigned long long " << var << " = " << init << ";\n";
+          if (by_warp) {
+            o << "    { const unsigned long long y_ = " << value("0") << "; " << var << " = cx::" << warp_fn << "(y_); }\n";
+          } else {
+            o << "    for (int r = 0; r < " << LREP << "; ++r) { const unsigned long long y_ = " << value("r") << "; " << fold << " }\n";
+          }
+        };
+        auto at = [&](int w, const std::string& r) { return "w_[" + std::to_string(w * LREP) + " + " + r + "]"; };
+        auto u64 = [&](int w) {
+          return [=](const std::string& r) { return "cx::lohi(" + at(w, r) + ", " + at(w + 1, r) + ")"; };
+        };
+        auto u32 = [&](int w) {
+          return [=](const std::string& r) { return "(unsigned long long)" + at(w, r); };
+        };
+        const std::string v = "v" + std::to_string(k) + "_", c = "c" + std::to_string(k) + "_";
+        const int w0 = w32_word[k];
+        if (f == AggFn::Min || f == AggFn::Max) {
+          auto val = [=](const std::string& r) { return "(unsigned long long)(long long)(int)" + at(w0, r); };
+          if (f == AggFn::Min) reduce(v, "~0ULL", v + " = y_ < " + v + " ? y_ : " + v + ";", "warp_min_u64", val);
+          else reduce(v, "0ULL", v + " = y_ > " + v + " ? y_ : " + v + ";", "warp_max_u64", val);
+        } else if (f == AggFn::Count) {
+          if (cnt_words == 2) reduce(v, "0ULL", v + " += y_;", "warp_sum_u64", u64(w0));
+          else reduce(v, "0ULL", v + " += y_;", "warp_sum_u64", u32(w0));
+        } else {
+          reduce(v, "0ULL", v + " += y_;", "warp_sum_u64", u64(w0));
+          if (f == AggFn::Avg) {
+            if (cnt_words == 2) reduce(c, "0ULL", c + " += y_;", "warp_sum_u64", u64(w0 + 2));
+            else reduce(c, "0ULL", c + " += y_;", "warp_sum_u64", u32(w0 + 2));
+          }
+        }
+      }
+      if (star_slot >= 0) o << "    if (v" << star_slot - (int)p.groups.size() << "_ == 0ULL) continue;\n";
+      if (by_warp) o << "    if (lane != 0) continue;\n";
+      emit_key_store(o, "g", "    ");
+      for (int k = 0; k < NA; ++k) {
+        const AggFn f = p.aggs[k].fn;
+        const std::string v = "v" + std::to_string(k) + "_";
+        const std::string ix = "(unsigned long long)g * " + std::to_string(TS) + "ULL + " + std::to_string((int)p.groups.size() + k);
+        if (f == AggFn::Min) o << "    if (" << v << " != ~0ULL) atomicMin(&d_result[" << ix << "], " << v << ");\n";
+        else if (f == AggFn::Max) o << "    if (" << v << " != 0ULL) atomicMax(&d_result[" << ix << "], " << v << ");\n";
+        else o << "    if (" << v << " != 0ULL) atomicAdd(&d_result[" << ix << "], " << v << ");\n";
+        if (!p.sparse) {
+          if (f == AggFn::Count) o << "    db::atomic_set_valid_bit(d_result_validity, " << ix << ");\n";
+          if (seen_idx[k] >= 0)
+            o << "    if ((s_seen[" << (unsigned long long)seen_idx[k] * TW << "u + (g >> 5)] >> (g & 31)) & 1u) db::atomic_set_valid_bit(d_result_validity, " << ix << ");\n";
+        }
+        if (f == AggFn::Avg)
+          o << "    if (c" << k << "_ != 0ULL) atomicAdd(&d_result[(unsigned long long)g * " << TS << "ULL + " << p.hidden_count_slot(k) << "], c" << k << "_);\n";
+      }
       o << "  }\n";
     } else if (smem_groups) {
       o << "  __syncthreads();\n";
