@@ -970,7 +970,7 @@ struct Emitter {
       for (int k = 0; k < NA; ++k)
         if (seen_idx[k] >= 0 && NSEEN_T > 0) o << "  unsigned rseen_" << k << " = 0u;\n";
     } else if (w32) {
-      o << "  unsigned int* s_w32 = (unsigned int*)(cx_smem + " << acc_off << ");\n";
+      o << "  unsigned int* cx_w32 = (unsigned int*)(cx_smem + " << acc_off << ");\n";
       o << "  unsigned int* s_touch = (unsigned int*)(cx_smem + " << touch_off << "); (void)s_touch;\n";
       o << "  unsigned int* s_seen = (unsigned int*)(cx_smem + " << seen_off << "); (void)s_seen;\n";
       std::string min_words;
@@ -978,7 +978,7 @@ struct Emitter {
         if (p.aggs[k].fn == AggFn::Min) min_words += (min_words.empty() ? "" : " || ") + std::string("s == ") + std::to_string(w32_word[k]);
       o << "  for (unsigned w = threadIdx.x; w < " << G * W32 * LREP << "u; w += " << CTA << ") {\n";
       if (!min_words.empty()) o << "    const unsigned s = w / " << LREP << "u % " << W32 << "u;\n";
-      o << "    s_w32[w] = " << (min_words.empty() ? "0u" : "(" + min_words + ") ? ~0u : 0u") << ";\n";
+      o << "    cx_w32[w] = " << (min_words.empty() ? "0u" : "(" + min_words + ") ? ~0u : 0u") << ";\n";
       o << "  }\n";
       o << "  for (unsigned w = threadIdx.x; w < " << TW * (1 + NSEEN_T) << "u; w += " << CTA << ") s_touch[w] = 0u;\n";
     } else if (smem_groups) {
@@ -1314,7 +1314,7 @@ struct Emitter {
       auto set_bit = [&](const std::string& words) {
         o << ii << "cx::set_bit_once(&" << words << ", 1u << (hash & 31));\n";
       };
-      o << ii << "unsigned* w_ = s_w32 + (unsigned)hash * " << W32 * LREP << "u"
+      o << ii << "unsigned* w_ = cx_w32 + (unsigned)hash * " << W32 * LREP << "u"
         << (LREP > 1 ? " + (lane & " + std::to_string(LREP - 1) + ")" : std::string()) << ";\n";
       if (star_slot < 0) set_bit("s_touch[hash >> 5]");
       for (int k = 0; k < NA; ++k) {
@@ -1373,10 +1373,10 @@ struct Emitter {
         // The OR-join's probes are done (or_probes): each branch is a hit bit.
         for (size_t f = 0; f < j.fks.size(); ++f) {
           const std::string F = std::to_string(f);
-          o << ii << "if ((or_hit_ >> (i * " << j.fks.size() << " + " << F << ")) & 1u) {\n";
-          if (!j.payload.empty()) o << ii << "  " << j.payload << "[i] = or_pay" << F << "_[i];\n";
+          o << ii << "if ((cx_or_hit >> (i * " << j.fks.size() << " + " << F << ")) & 1u) {\n";
+          if (!j.payload.empty()) o << ii << "  " << j.payload << "[i] = cx_or_pay" << F << "_[i];\n";
           if (!j.payload.empty() && payload_valid.count(j.payload))
-            o << ii << "  " << j.payload << "_valid[i] = (int)((or_val" << F << "_ >> i) & 1u);\n";
+            o << ii << "  " << j.payload << "_valid[i] = (int)((cx_or_val" << F << "_ >> i) & 1u);\n";
           item_steps(k + 1, ii + "  ");
           o << ii << "}\n";
         }
@@ -1629,10 +1629,10 @@ struct Emitter {
       const std::string ht = ht_name(j.dim);
       const size_t F = j.fks.size();
       const bool pay = !j.payload.empty(), pv_pay = pay && payload_valid.count(j.payload);
-      o << ii << (IPT * F > 32 ? "unsigned long long" : "unsigned") << " or_hit_ = 0u;\n";
+      o << ii << (IPT * F > 32 ? "unsigned long long" : "unsigned") << " cx_or_hit = 0u;\n";
       for (size_t f = 0; f < F; ++f) {
-        if (pay) o << ii << "int or_pay" << f << "_[ITEMS_PER_THREAD];\n";
-        if (pv_pay) o << ii << "unsigned or_val" << f << "_ = 0u;\n";
+        if (pay) o << ii << "int cx_or_pay" << f << "_[ITEMS_PER_THREAD];\n";
+        if (pv_pay) o << ii << "unsigned cx_or_val" << f << "_ = 0u;\n";
       }
       for (size_t f = 0; f < F; ++f) {
         const std::string& fk = j.fks[f];
@@ -1643,20 +1643,20 @@ struct Emitter {
           terms.push_back(lit_true(pv) ? fk + "[i] != " + pf + "[i]" : "(!(" + pv + ") || " + fk + "[i] != " + pf + "[i])");
         }
         o << ii << "#pragma unroll\n" << ii << "for (int i = 0; i < ITEMS_PER_THREAD; ++i) {\n";
-        o << ii << "  const int h_ = (" << and_terms(terms) << ") ? cx_detail::pht_slot<int>(" << fk << "[i], " << j.len << ", " << j.keymin
+        o << ii << "  const int cx_h = (" << and_terms(terms) << ") ? cx_detail::pht_slot<int>(" << fk << "[i], " << j.len << ", " << j.keymin
           << ") : -1;\n";
         if (pay) {
-          o << ii << "  int2 kv_ = make_int2(0, 0);\n";
-          o << ii << "  if (h_ >= 0) kv_ = ((const int2*)" << ht << ")[h_];\n";
-          o << ii << "  or_pay" << f << "_[i] = kv_.y;\n";
+          o << ii << "  int2 cx_kv = make_int2(0, 0);\n";
+          o << ii << "  if (cx_h >= 0) cx_kv = ((const int2*)" << ht << ")[cx_h];\n";
+          o << ii << "  cx_or_pay" << f << "_[i] = cx_kv.y;\n";
         } else {
-          o << ii << "  int2 kv_ = make_int2(0, 0);\n";
-          o << ii << "  if (h_ >= 0) kv_.x = " << ht << "[h_];\n";
+          o << ii << "  int2 cx_kv = make_int2(0, 0);\n";
+          o << ii << "  if (cx_h >= 0) cx_kv.x = " << ht << "[cx_h];\n";
         }
-        o << ii << "  const bool hit_ = h_ >= 0 && kv_.x == " << fk << "[i];\n";
-        o << ii << "  or_hit_ |= (" << (IPT * F > 32 ? "unsigned long long" : "unsigned") << ")hit_ << (i * " << F << " + " << f << ");\n";
+        o << ii << "  const bool hit_ = cx_h >= 0 && cx_kv.x == " << fk << "[i];\n";
+        o << ii << "  cx_or_hit |= (" << (IPT * F > 32 ? "unsigned long long" : "unsigned") << ")hit_ << (i * " << F << " + " << f << ");\n";
         if (pv_pay)
-          o << ii << "  if (hit_) or_val" << f << "_ |= ((" << ht << "_valid[h_ >> 5] >> (h_ & 31)) & 1u) << i;\n";
+          o << ii << "  if (hit_) cx_or_val" << f << "_ |= ((" << ht << "_valid[cx_h >> 5] >> (cx_h & 31)) & 1u) << i;\n";
         o << ii << "}\n";
       }
     };
@@ -1852,7 +1852,7 @@ struct Emitter {
       if (by_warp) o << "  for (int g = warp; g < " << G << "; g += NWARP) {\n";
       else o << "  for (int g = threadIdx.x; g < " << G << "; g += " << CTA << ") {\n";
       if (star_slot < 0) o << "    if (!((s_touch[g >> 5] >> (g & 31)) & 1u)) continue;\n";
-      o << "    const unsigned* w_ = s_w32 + (unsigned)g * " << W32 * LREP << "u" << (by_warp ? " + lane" : "") << ";\n";
+      o << "    const unsigned* w_ = cx_w32 + (unsigned)g * " << W32 * LREP << "u" << (by_warp ? " + lane" : "") << ";\n";
       for (int k = 0; k < NA; ++k) {
         const Agg& ag = p.aggs[k];
         const AggFn f = ag.fn;
