@@ -532,6 +532,48 @@ CX_DEVICE void BlockBuildSelectivePHT_2V(int tid, K (&keys)[ITEMS_PER_THREAD], V
     }
   });
 }
+// Build of a PHT_1 (WORDS 1) or PHT_2 (WORDS 2; with `ht_valid`, a PHT_2V)
+// together with its exact membership bitmap: bit h set when slot h holds the
+// in-window key key_min + h.  A slot's key never changes once it is taken, so
+// the row whose compare-and-swap found it empty or its own key settles the bit
+// for good.  Key 0 leaves its slot empty; the scan decides that bit.  All
+// threads of the block call it (ballots): rows of a tile are mostly
+// neighbouring keys, so each warp sets two words, not 32 bits one by one.
+// No counterpart in the reference API.
+template <int WORDS, int BLOCK_THREADS, int ITEMS_PER_THREAD>
+CX_DEVICE void BlockBuildMarkedPHT(int tid, int (&keys)[ITEMS_PER_THREAD], int (&vals)[ITEMS_PER_THREAD],
+                                   int (&vals_valid)[ITEMS_PER_THREAD], int (&flags)[ITEMS_PER_THREAD], int* ht,
+                                   unsigned int* ht_valid, unsigned int* bm, int ht_len, int key_min, int num_items) {
+#pragma unroll
+  for (int i = 0; i < ITEMS_PER_THREAD; ++i) {
+    int h = -1;
+    bool mark = false;
+    if (i * BLOCK_THREADS + tid < num_items && flags[i]) {
+      h = cx_detail::pht_slot<int>(keys[i], ht_len, key_min);
+      if (h >= 0) {
+        const int prev = atomicCAS(&ht[(long long)h * WORDS], 0, keys[i]);
+        if (prev == 0 || prev == keys[i]) {
+          if (WORDS == 2) {
+            ht[2LL * h + 1] = vals[i];
+            if (ht_valid && vals_valid[i]) atomicOr(&ht_valid[h >> 5], 1u << (h & 31));
+          }
+          mark = keys[i] != 0 && keys[i] == (int)((long long)key_min + h);
+        }
+      }
+    }
+    unsigned left = __ballot_sync(0xffffffffu, mark);
+    for (int round = 0; round < 2 && left; ++round) {
+      const int w = __shfl_sync(0xffffffffu, h >> 5, __ffs(left) - 1);
+      const bool mine = mark && (h >> 5) == w;
+      const unsigned bits = __reduce_or_sync(0xffffffffu, mine ? 1u << (h & 31) : 0u);
+      const unsigned took = __ballot_sync(0xffffffffu, mine);
+      if ((threadIdx.x & 31) == 0) atomicOr(&bm[w], bits);
+      if (mine) mark = false;
+      left &= ~took;
+    }
+    if (mark) atomicOr(&bm[h >> 5], 1u << (h & 31));
+  }
+}
 template <typename K, typename V, int BLOCK_THREADS, int ITEMS_PER_THREAD>
 CX_DEVICE void BlockProbeAndPHT_2V(int tid, K (&items)[ITEMS_PER_THREAD], V (&res)[ITEMS_PER_THREAD],
                                    int (&res_valid)[ITEMS_PER_THREAD], int (&flags)[ITEMS_PER_THREAD], const K* ht,
@@ -862,6 +904,29 @@ CX_DEVICE unsigned long long warp_max_u64(unsigned long long x) {
     x = y > x ? y : x;
   }
   return x;
+}
+
+// Blocks of a build over `rows` rows: one per `tile` rows, at most `cap` (each
+// then takes several tiles).  The host sizes the grid by the same rule.
+CX_DEVICE long long build_blocks(long long rows, int tile, int cap) {
+  const long long n = (rows + tile - 1) / tile;
+  return n < cap ? n : cap;
+}
+
+// ProbeMultiHT over the generated build's directory of four ints per slot
+// (key, offset, count, and the build's write cursor): one 16-byte load.
+CX_DEVICE void ProbeMultiHT4(int key, int& offset, int& count, int& flag, const int* ht_dir, int ht_len, int key_min) {
+  count = 0;
+  if (!flag) return;
+  const int h = cx_detail::pht_slot<int>(key, ht_len, key_min);
+  int4 e = make_int4(0, 0, 0, 0);
+  if (h >= 0) e = reinterpret_cast<const int4*>(ht_dir)[h];
+  if (h >= 0 && e.x == key && e.z > 0) {
+    offset = e.y;
+    count = e.z;
+  } else {
+    flag = 0;
+  }
 }
 
 CX_DEVICE unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }

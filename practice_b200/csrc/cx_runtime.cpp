@@ -104,6 +104,8 @@ struct KernelSpec {
   std::string name, kind;
   int table = 0, block = 128, tile = 512, ctas_per_sm = 1;
   size_t smem = 0;
+  int cap = 0;                // "builds": most blocks of one table
+  std::vector<int> parts;     // "builds": tables, each with its own range of blocks
 };
 
 struct LaunchPlan {
@@ -272,7 +274,16 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
       KernelSpec ks;
       ls >> ks.name >> ks.kind >> ks.table >> ks.block;
       if (ks.kind == "build" || ks.kind == "cubeidx" || ks.kind == "tiles" || ks.kind == "tilescan") ls >> ks.tile;
-      else if (ks.kind == "scan" || ks.kind == "sharedscan" || ks.kind == "cubescan") ls >> ks.tile >> ks.smem >> ks.ctas_per_sm;
+      else if (ks.kind == "builds") {
+        size_t n = 0;
+        ls >> ks.tile >> ks.cap >> n;
+        for (size_t i = 0; i < n && ls; ++i) {
+          int t = -1;
+          ls >> t;
+          ks.parts.push_back(t);
+        }
+      } else if (ks.kind == "prep") {
+      } else if (ks.kind == "scan" || ks.kind == "sharedscan" || ks.kind == "cubescan") ls >> ks.tile >> ks.smem >> ks.ctas_per_sm;
       else { size_t z; ls >> z; }
       lp.kernels.push_back(ks);
     } else {
@@ -296,6 +307,15 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
       err = "kernel line " + k.name + " names a table outside the plan or a bad shape";
       return false;
     }
+  for (const auto& k : lp.kernels) {
+    if (k.kind != "builds") continue;
+    bool ok = k.tile > 0 && k.block > 0 && k.block <= 1024 && k.cap > 0 && !k.parts.empty();
+    for (int t : k.parts) ok = ok && t >= 0 && t < (int)lp.tables.size();
+    if (!ok) {
+      err = "kernel line " + k.name + " names a table outside the plan or a bad shape";
+      return false;
+    }
+  }
   return true;
 }
 
@@ -1316,11 +1336,21 @@ int cx_execute_params(cx_module* m, cx_exec_ctx* c, const int32_t* params, int n
     return CX_OK;
   };
 
+  a.zero_base = (unsigned char*)scratch;
+  a.zero_bytes = (long long)sl.total;
   CX_CUDA(cudaEventRecord(c->ev[0], stream));
-  CX_CUDA(cudaMemsetAsync(scratch, 0, sl.total, stream));
-  CX_CUDA(cudaMemsetAsync(c->result, 0, lp.result_words * 8, stream));
-  CX_CUDA(cudaMemsetAsync(c->validity, 0, vwords * 8, stream));
   size_t ki = 0;
+  if (!lp.kernels.empty() && lp.kernels[0].kind == "prep") {
+    // One kernel for all of it, a thread per 16 bytes up to four CTAs per SM.
+    const KernelSpec& k = lp.kernels[0];
+    const uint64_t vecs = (sl.total + lp.result_words * 8 + vwords * 8 + 15) / 16;
+    if ((rc = launch(0, (unsigned)std::min<uint64_t>((vecs + k.block - 1) / k.block, (uint64_t)sms * 4)))) return rc;
+    ++ki;
+  } else {
+    CX_CUDA(cudaMemsetAsync(scratch, 0, sl.total, stream));
+    CX_CUDA(cudaMemsetAsync(c->result, 0, lp.result_words * 8, stream));
+    CX_CUDA(cudaMemsetAsync(c->validity, 0, vwords * 8, stream));
+  }
   // Phase 1: slot initialisation and hash-table builds.
   for (; ki < lp.kernels.size() && lp.kernels[ki].kind != "scan" && lp.kernels[ki].kind != "tilescan"; ++ki) {
     const KernelSpec& k = lp.kernels[ki];
@@ -1330,6 +1360,8 @@ int cx_execute_params(cx_module* m, cx_exec_ctx* c, const int32_t* params, int n
     else if (k.kind == "build") {
       const long long tiles = (rows[k.table] + k.tile - 1) / k.tile;
       grid = (unsigned)std::min<long long>(tiles, (long long)sms * 16);
+    } else if (k.kind == "builds") {
+      for (int t : k.parts) grid += (unsigned)std::min<long long>((rows[t] + k.tile - 1) / k.tile, k.cap);
     } else if (k.kind == "tiles") {
       // One CTA per tile of the table (a translated nd_range kernel).
       grid = (unsigned)((rows[k.table] + k.tile - 1) / k.tile);
