@@ -197,10 +197,14 @@ def translate_visitor(source: str) -> str:
 def plan_literals(plan_text: str) -> list[int]:
     raw = plan_text.encode()
     n = C.c_int(0)
-    check(lib.cx_plan_literals(raw, len(raw), None, 0, C.byref(n)), "cx_plan_literals")
-    out = (C.c_int64 * max(n.value, 1))()
-    check(lib.cx_plan_literals(raw, len(raw), out, n.value, C.byref(n)), "cx_plan_literals")
-    return list(out[: n.value])
+    cap = 256  # one call, one parse, for all but the longest plans
+    while True:
+        out = (C.c_int64 * cap)()
+        rc = lib.cx_plan_literals(raw, len(raw), out, cap, C.byref(n))
+        if rc != -5 or n.value <= cap:  # CX_E_CAPACITY
+            check(rc, "cx_plan_literals")
+            return out[: n.value]
+        cap = n.value
 
 
 def shared_codegen(plan_texts: list[str], tuning: Tuning | None = None) -> str:

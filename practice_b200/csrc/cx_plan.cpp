@@ -7,6 +7,7 @@
 #include <cstring>
 #include <functional>
 #include <set>
+#include <unordered_set>
 
 namespace cx {
 
@@ -96,7 +97,7 @@ const std::string& to_name(const Node& n, const char* what) {
 // library's primitives, or one of the generated code's own identifiers
 // (fixed names, and numbered temporaries such as gt3 or x5_).
 void check_column_name(const std::string& c) {
-  static const std::set<std::string> reserved = {
+  static const std::unordered_set<std::string> reserved = {
       // C++ keywords
       "alignas", "alignof", "and", "and_eq", "asm", "auto", "bitand", "bitor", "bool", "break", "case", "catch",
       "char", "char8_t", "char16_t", "char32_t", "class", "compl", "concept", "const", "consteval", "constexpr",
@@ -147,6 +148,7 @@ void check_column_name(const std::string& c) {
       c.compare(0, 3, "CX_") == 0 || c.compare(0, 2, "__") == 0)
     bad("collides with this library's primitives");
   // Numbered temporaries: a short stem, digits, optionally _digits and a trailing underscore.
+  if (!std::isdigit((unsigned char)c.back()) && c.back() != '_') return;
   static const char* stems[] = {"gt", "gd", "x", "v", "h", "k", "e", "w", "g", "cl", "o", "j", "b", "s", "at",
                                 "off", "acc_", "seen_", "t", "c", "l", "fb", "fw", "m", "p", "r", "q", "y", "z"};
   for (const char* st : stems) {

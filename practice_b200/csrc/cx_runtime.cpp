@@ -14,6 +14,7 @@
 #include <nvrtc.h>
 
 #include <atomic>
+#include <cstddef>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -404,7 +405,11 @@ struct cx_module {
   // once per cube layout with the layout as constants, per layout and device.
   std::string source;
   struct Spec { CUmodule mod = nullptr; CUfunction fn = nullptr; bool failed = false; };
-  std::map<std::string, std::map<int, Spec>> cube_specs;
+  // The layout values the cube region reads (its `#define CXS_*` lines), found
+  // once at compile; a batch's layout is their values in this order.
+  struct CubeHook { std::string name; size_t off; bool wide; };
+  std::vector<CubeHook> cube_hooks;
+  std::map<std::vector<long long>, std::map<int, Spec>> cube_specs;
 };
 
 struct cx_exec_ctx {
@@ -482,6 +487,55 @@ int load_on_device(cx_module* m, int dev, cx_module::Loaded** out) {
   return CX_OK;
 }
 
+// The layout hooks of a shared program's cube region: its default lines
+// "#define NAME (a.field[idx])" or "#define NAME (a.field)", each as the place
+// of its value in the kernel arguments.  Empty if a line has another form (the
+// generic kernel then always runs).
+std::vector<cx_module::CubeHook> cube_hooks_of(const std::string& src) {
+  struct Field { const char* name; size_t off; int n; bool wide; };
+  static const Field fields[] = {
+      {"cube_dsm_bytes", offsetof(CxArgs, cube_dsm_bytes), 0, false},
+      {"cube_smem_words", offsetof(CxArgs, cube_smem_words), 0, false},
+      {"cube_dsm", offsetof(CxArgs, cube_dsm), CX_MAX_HTS, false},
+      {"cube_dgl", offsetof(CxArgs, cube_dgl), CX_MAX_HTS, false},
+      {"cube_desz", offsetof(CxArgs, cube_desz), CX_MAX_HTS, false},
+      {"cube_dbase", offsetof(CxArgs, cube_dbase), CX_MAX_HTS, false},
+      {"cube_dlen", offsetof(CxArgs, cube_dlen), CX_MAX_HTS, false},
+      {"cube_fsh", offsetof(CxArgs, cube_fsh), CX_MAX_HTS * 4, false},
+      {"cube_fmk", offsetof(CxArgs, cube_fmk), CX_MAX_HTS * 4, false},
+      {"cube_stride", offsetof(CxArgs, cube_stride), CX_MAX_SHAPES * CX_MAX_SATTRS, false},
+      {"cube_smem", offsetof(CxArgs, cube_smem), CX_MAX_SHAPES, false},
+      {"cube_cells", offsetof(CxArgs, cube_cells), CX_MAX_SHAPES, true},
+      {"cube_lo", offsetof(CxArgs, cube_lo), CX_MAX_CATTRS, false},
+      {"cube_radix", offsetof(CxArgs, cube_radix), CX_MAX_CATTRS, false}};
+  std::vector<cx_module::CubeHook> hooks;
+  const size_t r0 = src.find("//@cx-cube-begin"), r1 = src.find("//@cx-cube-end");
+  if (r0 == std::string::npos || r1 == std::string::npos) return hooks;
+  std::istringstream in(src.substr(r0, r1 - r0));
+  std::string line;
+  while (std::getline(in, line)) {
+    if (line.rfind("#define CXS_", 0) != 0) continue;
+    std::istringstream ls(line);
+    std::string def, name, expr;
+    ls >> def >> name >> expr;
+    if (expr.size() < 5 || expr.compare(0, 3, "(a.") != 0) return {};
+    std::string body = expr.substr(3, expr.size() - 4);
+    int idx = 0;
+    const size_t lb = body.find('[');
+    const bool indexed = lb != std::string::npos;
+    if (indexed) {
+      idx = atoi(body.c_str() + lb + 1);
+      body = body.substr(0, lb);
+    }
+    const Field* f = nullptr;
+    for (const Field& k : fields)
+      if (body == k.name) f = &k;
+    if (!f || indexed != (f->n > 0) || (indexed && (idx < 0 || idx >= f->n))) return {};
+    hooks.push_back({name, f->off + (size_t)idx * (f->wide ? sizeof(long long) : sizeof(int)), f->wide});
+  }
+  return hooks;
+}
+
 // The cube scan of a shared program compiled with one batch layout as
 // constants: the program's prelude, `#define`s of the CXS_* layout macros
 // (values from the batch's arguments) and the program's cube region.  Cached
@@ -489,58 +543,24 @@ int load_on_device(cx_module* m, int dev, cx_module::Loaded** out) {
 // program has no cube region or the compile fails.
 int cube_spec_function(cx_module* m, int dev, const CxArgs& a, const std::string& kname, size_t smem_max, CUfunction* fn) {
   *fn = nullptr;
+  if (m->cube_hooks.empty()) return CX_OK;
+  std::vector<long long> layout;
+  layout.reserve(m->cube_hooks.size());
+  for (const auto& h : m->cube_hooks) {
+    const char* at = (const char*)&a + h.off;
+    layout.push_back(h.wide ? *(const long long*)at : *(const int*)at);
+  }
+  std::lock_guard<std::mutex> lk(m->mu);
+  cx_module::Spec& sp = m->cube_specs[layout][dev];
+  if (sp.fn || sp.failed) { *fn = sp.fn; return CX_OK; }
   const std::string& src = m->source;
   const size_t p0 = src.find("@*/"), p1 = src.find("//@cx-prelude-end");
   const size_t r0 = src.find("//@cx-cube-begin"), r1 = src.find("//@cx-cube-end");
-  if (p0 == std::string::npos || p1 == std::string::npos || r0 == std::string::npos || r1 == std::string::npos) return CX_OK;
-  std::string region = src.substr(r0, r1 - r0);
-  // Default lines: "#define NAME (a.field[idx])" or "#define NAME (a.field)".
-  std::string defs = "#define CXS_SPEC 1\n";
-  std::istringstream in(region);
-  std::string line;
-  auto value = [&](const std::string& f, int i, bool* ok) -> long long {
-    *ok = true;
-    auto in_range = [&](int n) { if (i < 0 || i >= n) *ok = false; return *ok; };
-    if (f == "cube_dsm_bytes") return a.cube_dsm_bytes;
-    if (f == "cube_smem_words") return a.cube_smem_words;
-    if (f == "cube_dsm" && in_range(CX_MAX_HTS)) return a.cube_dsm[i];
-    if (f == "cube_dgl" && in_range(CX_MAX_HTS)) return a.cube_dgl[i];
-    if (f == "cube_desz" && in_range(CX_MAX_HTS)) return a.cube_desz[i];
-    if (f == "cube_dbase" && in_range(CX_MAX_HTS)) return a.cube_dbase[i];
-    if (f == "cube_dlen" && in_range(CX_MAX_HTS)) return a.cube_dlen[i];
-    if (f == "cube_fsh" && in_range(CX_MAX_HTS * 4)) return a.cube_fsh[i];
-    if (f == "cube_fmk" && in_range(CX_MAX_HTS * 4)) return a.cube_fmk[i];
-    if (f == "cube_stride" && in_range(CX_MAX_SHAPES * CX_MAX_SATTRS)) return a.cube_stride[i];
-    if (f == "cube_smem" && in_range(CX_MAX_SHAPES)) return a.cube_smem[i];
-    if (f == "cube_cells" && in_range(CX_MAX_SHAPES)) return a.cube_cells[i];
-    if (f == "cube_lo" && in_range(CX_MAX_CATTRS)) return a.cube_lo[i];
-    if (f == "cube_radix" && in_range(CX_MAX_CATTRS)) return a.cube_radix[i];
-    *ok = false;
-    return 0;
-  };
-  while (std::getline(in, line)) {
-    if (line.rfind("#define CXS_", 0) != 0) continue;
-    std::istringstream ls(line);
-    std::string def, name, expr;
-    ls >> def >> name >> expr;
-    // expr: "(a.field[idx])" or "(a.field)"
-    if (expr.size() < 5 || expr.compare(0, 3, "(a.") != 0) return CX_OK;
-    std::string body = expr.substr(3, expr.size() - 4);
-    int idx = -1;
-    const size_t lb = body.find('[');
-    if (lb != std::string::npos) {
-      idx = atoi(body.c_str() + lb + 1);
-      body = body.substr(0, lb);
-    }
-    bool ok = false;
-    const long long v = value(body, idx, &ok);
-    if (!ok) return CX_OK;
-    defs += "#define " + name + " (" + std::to_string(v) + (body == "cube_cells" ? "LL" : "") + ")\n";
-  }
-  std::lock_guard<std::mutex> lk(m->mu);
-  cx_module::Spec& sp = m->cube_specs[defs][dev];
-  if (sp.fn || sp.failed) { *fn = sp.fn; return CX_OK; }
-  const std::string prog_src = src.substr(p0 + 3, p1 - p0 - 3) + "\n" + defs + region;
+  if (p0 == std::string::npos || p1 == std::string::npos) { sp.failed = true; return CX_OK; }
+  std::string prog_src = src.substr(p0 + 3, p1 - p0 - 3) + "\n#define CXS_SPEC 1\n";
+  for (size_t i = 0; i < layout.size(); ++i)
+    prog_src += "#define " + m->cube_hooks[i].name + " (" + std::to_string(layout[i]) + (m->cube_hooks[i].wide ? "LL" : "") + ")\n";
+  prog_src += src.substr(r0, r1 - r0);
   nvrtcProgram prog;
   const char* headers[] = {kCxEmbeddedCrystalHeader, kCxEmbeddedArgsHeader};
   const char* names[] = {"crystal_sm100.cuh", "cx_args.h"};
@@ -1064,7 +1084,10 @@ int cx_compile(const char* src, size_t src_len, const char* key, cx_module** out
   std::string perr;
   if (!parse_launch_plan(source, m->lp, perr)) return fail(CX_E_INVALID, "cx_compile: %s", perr.c_str());
   m->sl = scratch_layout(m->lp);
-  if (m->lp.cube) m->source = source;
+  if (m->lp.cube) {
+    m->source = source;
+    m->cube_hooks = cube_hooks_of(source);
+  }
 
   nvrtcProgram prog;
   const char* headers[] = {kCxEmbeddedCrystalHeader, kCxEmbeddedArgsHeader};

@@ -59,6 +59,11 @@ def shape_key(plan: Plan) -> str:
     return plan.memo("shape", lambda: re.sub(r"\(int -?\d+\)", "(int ?)", plan.text()))
 
 
+def plan_literals(plan: Plan) -> list[int]:
+    """The plan's literals, parsed once per plan (a plan is not changed in place)."""
+    return plan.memo("literals", lambda: _lib.plan_literals(plan.text()))
+
+
 DEFAULT_CANDIDATES = [
     dict(block_threads=bt, items_per_thread=ipt, stages=st, ctas_per_sm=cs)
     for bt, ipt, st, cs in itertools.product((256, 512, 1024), (2, 4, 8), (0, 2, 4), (1, 16))
@@ -309,7 +314,7 @@ class Database:
         for p, (words, ro, rw, vo, vw) in zip(plans, lay):
             s = prog.index[shape_key(p)]
             res, val = arena[ro:ro + rw], arena[vo:vo + vw]
-            lits = _lib.plan_literals(p.text())
+            lits = plan_literals(p)
             queries.append(_lib.SharedQuery(s, len(params), res.data_ptr(), res.numel(), val.data_ptr(), val.numel()))
             params.extend(lits)
             bufs.append((res, val, words))
@@ -339,9 +344,11 @@ class Database:
         out = []
         for res, val, words in bufs:
             ro, vo = (res.data_ptr() - base) // 8, (val.data_ptr() - base) // 8
-            w = host[ro:ro + words].copy()
-            v = host[vo:vo + (words + 63) // 64].copy()
-            out.append(QueryResult(w, v, timing, err))
+            w, v = host[ro:ro + words], host[vo:vo + (words + 63) // 64]
+            # Views of the batch's one host copy; from 1 MiB on each result gets
+            # its own, so that keeping one does not keep the whole batch.
+            out.append(QueryResult(w, v, timing, err) if host.nbytes < (1 << 20) else
+                       QueryResult(w.copy(), v.copy(), timing, err))
         return out
 
     def autotune_shared(self, plans: list[Plan], candidates: list[dict], reps: int = 2) -> dict:
@@ -409,12 +416,14 @@ class Database:
         torch = self.torch
         tuning = tuning if tuning is not None else self.tuning_for(plan)
         m = self.compile(plan, tuning)
-        res, val = self.alloc_result(m)
+        # Result words, then validity words, in one buffer: one copy brings both back.
+        rw, vw = max(int(m.info.result_words), 1), max(int(m.info.validity_words), 1)
+        buf = torch.empty(rw + vw, dtype=torch.int64, device=self.device)
         for t, n in self.rows.items():
             self.ctx.set_rows(t, n)
-        self.ctx.set_result(res.data_ptr(), res.numel(), val.data_ptr(), val.numel())
+        self.ctx.set_result(buf.data_ptr(), rw, buf.data_ptr() + 8 * rw, vw)
         s = stream if stream is not None else torch.cuda.current_stream()
-        params = _lib.plan_literals(plan.text()) if tuning is not None and tuning.parametric else None
+        params = plan_literals(plan) if tuning is not None and tuning.parametric else None
         self.ctx.execute(m, s.cuda_stream, params)
         err = 0
         try:
@@ -424,6 +433,5 @@ class Database:
                 raise
             err = self.ctx.kernel_error()
         fw = int(m.info.final_words)
-        words = res.cpu().numpy().view(np.uint64)[:fw].copy()
-        validity = val.cpu().numpy().view(np.uint64)[: (fw + 63) // 64].copy()
-        return QueryResult(words, validity, self.ctx.timing(), err)
+        host = buf.cpu().numpy().view(np.uint64)
+        return QueryResult(host[:fw], host[rw:rw + (fw + 63) // 64], self.ctx.timing(), err)
