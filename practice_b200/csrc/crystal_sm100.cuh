@@ -831,7 +831,9 @@ CX_DEVICE void atomic_max_ull(unsigned long long& t, unsigned long long v) { ato
 
 CX_DEVICE void atomic_set_valid_bit(uint64_t* bitmap, unsigned long long bit) {
   if (bitmap == nullptr) return;
-  atomicOr((unsigned long long*)&bitmap[bit >> 6], 1ULL << (bit & 63ULL));
+  // Tested first: many CTAs set the same bits, and atomics on one word queue.
+  const uint64_t m = 1ULL << (bit & 63ULL);
+  if (!(*(volatile uint64_t*)&bitmap[bit >> 6] & m)) atomicOr((unsigned long long*)&bitmap[bit >> 6], (unsigned long long)m);
 }
 CX_DEVICE int bitmap_valid_at(const uint64_t* bitmap, unsigned long long bit) {
   if (bitmap == nullptr) return 1;
@@ -862,6 +864,17 @@ CX_DEVICE void raise(unsigned int* err, unsigned int code) {
   if (err) atomicCAS(err, 0u, code);
 }
 
+// Sets the bits `mask` from bit `first` on (at most two words); false when all
+// of them were set already.
+CX_DEVICE bool set_valid_bits(uint64_t* bitmap, unsigned long long first, unsigned long long mask) {
+  uint64_t* w = bitmap + (first >> 6);
+  const unsigned sh = (unsigned)(first & 63ULL);
+  const unsigned long long lo = mask << sh, hi = sh ? mask >> (64u - sh) : 0ULL;
+  bool set = false;
+  if (lo & ~*(volatile uint64_t*)w) { atomicOr((unsigned long long*)w, lo); set = true; }
+  if (hi && (hi & ~*(volatile uint64_t*)(w + 1))) { atomicOr((unsigned long long*)(w + 1), hi); set = true; }
+  return set;
+}
 // Group tables of 32-bit shared-memory words (native atomics).
 // x into a (low, high) pair: the low word's carry goes into the high one, so
 // the pair is the sum modulo 2^64 in any order of adds.
