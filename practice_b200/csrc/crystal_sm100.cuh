@@ -890,6 +890,9 @@ CX_DEVICE unsigned long long lohi(unsigned lo, unsigned hi) { return ((unsigned 
 CX_DEVICE void set_bit_once(unsigned* word, unsigned bit) {
   if (!(*word & bit)) atomicOr(word, bit);
 }
+CX_DEVICE void set_bits_once(unsigned* word, unsigned bits) {
+  if (bits & ~*word) atomicOr(word, bits);
+}
 CX_DEVICE void min_word(unsigned* word, unsigned x) {
   if (x < *word) atomicMin(word, x);
 }

@@ -59,7 +59,7 @@ struct CxArgs {
   // Aggregate cubes of a shared-scan batch: per attribute the registered range
   // minimum and the number of values; per shape the cell stride of each of its
   // attributes, its cube in global memory (sums per SUM aggregate, then row
-  // counts) and the u64 offset of its per-CTA copy in shared memory (-1: none).
+  // counts, or without COUNT aggregates one presence bit per cell) and the u64 offset of its per-CTA copy in shared memory (-1: none).
   int cube_lo[CX_MAX_CATTRS];
   int cube_radix[CX_MAX_CATTRS];
   int cube_stride[CX_MAX_SHAPES * CX_MAX_SATTRS];
@@ -92,6 +92,10 @@ struct CxArgs {
   int cube_fmk[CX_MAX_HTS * 4];
   int cube_dsm_bytes;                          // shared-memory bytes of all compact dimension copies
   int cube_dgl[CX_MAX_HTS];                    // 1: compact words gathered from global memory instead
+  // Presence bits of shapes without COUNT whose cube is in global memory: per
+  // shape the u32 offset of its bits in shared memory (-1: in the cube itself).
+  int cube_pres[CX_MAX_SHAPES];
+  int cube_pres_words;                         // u32 words of all of them
   unsigned char* zero_base;                    // plain queries: the scratch an execute starts from zeroed
   long long zero_bytes;
 };

@@ -2696,7 +2696,9 @@ struct SharedGen {
     o << "  unsigned char* s_dim = cx_smem + " << fr_bytes << "; (void)s_dim;\n";
     o << "  unsigned long long* s_cube = (unsigned long long*)(cx_smem + " << fr_bytes << " + a.cube_dsm_bytes);\n";
     o << "  const int lane = threadIdx.x & 31;\n";
+    o << "  unsigned* s_pres = (unsigned*)(s_cube + a.cube_smem_words); (void)s_pres;\n";
     o << "  for (int w = threadIdx.x; w < a.cube_smem_words; w += " << CTA << ") s_cube[w] = 0ULL;\n";
+    o << "  for (int w = threadIdx.x; w < a.cube_pres_words; w += " << CTA << ") s_pres[w] = 0u;\n";
     // Compact dimension words into shared memory (16-byte copies; the arrays are padded to 16 bytes).
     for (size_t di = 0; di < dims.size(); ++di) {
       o << "  if (a.cube_dsm[" << di << "] >= 0) {\n";
@@ -2948,8 +2950,16 @@ struct SharedGen {
       o << "        const unsigned long long nc_ = (unsigned long long)a.cube_cells[" << s << "];\n";
       for (int k = 0; k < NS; ++k)
         o << "        { const unsigned long long x_ = " << xs[s][k] << "; if (h" << s << "_) atomicAdd(&cg_[" << k << "ULL * nc_], x_); }\n";
-      if (counts) o << "        if (h" << s << "_) atomicAdd(&cg_[" << NS << "ULL * nc_], 1ULL);\n";
-      else o << "        if (h" << s << "_) cg_[" << NS << "ULL * nc_] = 1ULL;\n";
+      if (counts) {
+        o << "        if (h" << s << "_) atomicAdd(&cg_[" << NS << "ULL * nc_], 1ULL);\n";
+      } else {
+        // Presence bits of a global cube: in shared memory while they fit (a
+        // store per row beside the sum's atomic doubled the L2 traffic), else
+        // in the cube's own bitmap; either way tested before they are set.
+        o << "        unsigned* pb_ = a.cube_pres[" << s << "] >= 0 ? s_pres + a.cube_pres[" << s << "] : (unsigned*)(a.cube_g[" << s << "] + " << NS
+          << "ULL * nc_);\n";
+        o << "        if (h" << s << "_) cx::set_bit_once(&pb_[cl" << s << "_ >> 5], 1u << (cl" << s << "_ & 31u));\n";
+      }
       o << "      }\n";
     }
     o << "    }\n";
@@ -2963,16 +2973,31 @@ struct SharedGen {
       o << "    const unsigned* cs_ = (const unsigned*)(s_cube + a.cube_smem[" << s << "]);\n";
       o << "    const unsigned nc_ = (unsigned)a.cube_cells[" << s << "];\n";
       o << "    unsigned long long* cg_ = a.cube_g[" << s << "];\n";
-      o << "    for (unsigned c = threadIdx.x; c < nc_; c += " << CTA << ") {\n";
-      o << "      const unsigned n_ = cs_[" << 2 * NS << "u * nc_ + c];\n";
+      const bool counts = (int)shapes[s]->aggs.size() > NS;
+      if (!counts) o << "    unsigned* pb_ = (unsigned*)(cg_ + " << NS << "ULL * nc_);\n";
+      // A warp takes 32 neighbouring cells, whose presence bits are one word.
+      o << "    for (unsigned b_ = threadIdx.x & ~31u; b_ < nc_; b_ += " << CTA << ") {\n";
+      o << "      const unsigned c = b_ + lane;\n";
+      o << "      const unsigned n_ = c < nc_ ? cs_[" << 2 * NS << "u * nc_ + c] : 0u;\n";
+      if (!counts) {
+        o << "      const unsigned m_ = __ballot_sync(0xffffffffu, n_ != 0u);\n";
+        o << "      if (lane == 0 && m_) cx::set_bits_once(&pb_[b_ >> 5], m_);\n";
+      }
       o << "      if (!n_) continue;\n";
-      if ((int)shapes[s]->aggs.size() > NS) o << "      atomicAdd(&cg_[" << NS << "ULL * nc_ + c], (unsigned long long)n_);\n";
-      else o << "      cg_[" << NS << "ULL * nc_ + c] = 1ULL;\n";
+      if (counts) o << "      atomicAdd(&cg_[" << NS << "ULL * nc_ + c], (unsigned long long)n_);\n";
       for (int k = 0; k < NS; ++k)
         o << "      { const unsigned long long v_ = ((unsigned long long)cs_[" << 2 * k + 1 << "u * nc_ + c] << 32) | cs_["
           << 2 * k << "u * nc_ + c]; if (v_) atomicAdd(&cg_[" << k << "ULL * nc_ + c], v_); }\n";
       o << "    }\n";
       o << "  }\n";
+      if (!counts) {
+        o << "  if (a.cube_smem[" << s << "] < 0 && a.cube_pres[" << s << "] >= 0 && a.sq_num[" << s << "] > 0) {\n";
+        o << "    const unsigned* sp_ = s_pres + a.cube_pres[" << s << "];\n";
+        o << "    unsigned* pb_ = (unsigned*)(a.cube_g[" << s << "] + " << NS << "ULL * (unsigned long long)a.cube_cells[" << s << "]);\n";
+        o << "    for (unsigned w = threadIdx.x; w < (unsigned)((a.cube_cells[" << s << "] + 31) / 32); w += " << CTA << ")\n";
+        o << "      if (sp_[w]) cx::set_bits_once(&pb_[w], sp_[w]);\n";
+        o << "  }\n";
+      }
     }
     o << "}\n\n";
     // The batch's cube layout (dimension words, strides, cube offsets and
@@ -2986,7 +3011,7 @@ struct SharedGen {
         {"a.cube_dbase[", "CXS_DBASE"}, {"a.cube_dlen[", "CXS_DLEN"}, {"a.cube_fsh[", "CXS_FSH"},
         {"a.cube_fmk[", "CXS_FMK"}, {"a.cube_stride[", "CXS_STRIDE"}, {"a.cube_smem[", "CXS_SMEM"},
         {"a.cube_cells[", "CXS_CELLS"}, {"a.cube_lo[", "CXS_LO"}, {"a.cube_radix[", "CXS_RADIX"}, {"a.cube_dgl[", "CXS_DGL"},
-        {"a.cube_smem_words", "CXS_SMEMW"}};
+        {"a.cube_smem_words", "CXS_SMEMW"}, {"a.cube_pres_words", "CXS_PRESW"}, {"a.cube_pres[", "CXS_PRES"}};
     std::set<std::string> used;
     std::string out;
     for (size_t i = 0; i < body.size();) {
@@ -3025,6 +3050,8 @@ struct SharedGen {
   // Per query: the cells of its shape's cube that its predicates accept, added
   // into its result the way the per-query path adds rows (touched bits,
   // validity), each block taking one chunk of the cells.
+  static constexpr int CHUNK_CELLS = 2048;  // cells of one answer block: 8 per thread, so that decoding
+                                            // them (a division per attribute) is spread over the GPU
   void emit_cube_answer() {
     meta << "kernel cube_answer cubeans 0 256 0\n";
     std::ostringstream& o = src;
@@ -3052,11 +3079,18 @@ struct SharedGen {
       }
       o << "      const unsigned long long* cg_ = a.cube_g[" << s << "];\n";
       o << "      const long long nc_ = a.cube_cells[" << s << "];\n";
-      o << "      const long long per_ = (nc_ + nch - 1) / nch, c0_ = (long long)ch * per_;\n";
+      // As many chunks as the shape's own cells want, of at most nch.
+      o << "      const int ns_ = (int)((nc_ + " << CHUNK_CELLS << " - 1) / " << CHUNK_CELLS << " < nch ? (nc_ + " << CHUNK_CELLS << " - 1) / " << CHUNK_CELLS << " : nch);\n";
+      o << "      if (ch >= ns_) return;\n";
+      o << "      const long long per_ = (nc_ + ns_ - 1) / ns_, c0_ = (long long)ch * per_;\n";
       o << "      const long long c1_ = c0_ + per_ < nc_ ? c0_ + per_ : nc_;\n";
       o << "      for (long long c = c0_ + threadIdx.x; c < c1_; c += blockDim.x) {\n";
-      o << "        const unsigned long long n_ = cg_[" << NS << "ULL * (unsigned long long)nc_ + c];\n";
-      o << "        if (!n_) continue;\n";
+      if ((int)p.aggs.size() > NS) {
+        o << "        const unsigned long long n_ = cg_[" << NS << "ULL * (unsigned long long)nc_ + c];\n";
+        o << "        if (!n_) continue;\n";
+      } else {
+        o << "        if (!((((const unsigned*)(cg_ + " << NS << "ULL * (unsigned long long)nc_))[c >> 5] >> (c & 31)) & 1u)) continue;\n";
+      }
       o << "        const unsigned cu_ = (unsigned)c;\n";
       // Value offsets from the cell index; an attribute with a functional
       // source (stride 0) reads its offset from the source's through its table.

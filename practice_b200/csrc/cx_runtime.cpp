@@ -505,6 +505,8 @@ std::vector<cx_module::CubeHook> cube_hooks_of(const std::string& src) {
       {"cube_fmk", offsetof(CxArgs, cube_fmk), CX_MAX_HTS * 4, false},
       {"cube_stride", offsetof(CxArgs, cube_stride), CX_MAX_SHAPES * CX_MAX_SATTRS, false},
       {"cube_smem", offsetof(CxArgs, cube_smem), CX_MAX_SHAPES, false},
+      {"cube_pres_words", offsetof(CxArgs, cube_pres_words), 0, false},
+      {"cube_pres", offsetof(CxArgs, cube_pres), CX_MAX_SHAPES, false},
       {"cube_cells", offsetof(CxArgs, cube_cells), CX_MAX_SHAPES, true},
       {"cube_lo", offsetof(CxArgs, cube_lo), CX_MAX_CATTRS, false},
       {"cube_radix", offsetof(CxArgs, cube_radix), CX_MAX_CATTRS, false}};
@@ -614,7 +616,8 @@ struct CubePlan {
   std::vector<uint64_t> cells, goff;
   std::vector<std::vector<int>> stride;
   std::vector<int> smem_off;
-  uint64_t smem_words = 0, gbytes = 0;
+  std::vector<int> pres_off;             // shared-memory presence bits of a global cube (u32 offset, -1: none)
+  uint64_t smem_words = 0, pres_words = 0, gbytes = 0;
   int chunks = 1;
   std::vector<std::vector<int>> fdsrc;   // per shape and attribute position: source position, -1 none
   std::vector<const int*> fdtab;          // per attribute: its table from the source's value offset
@@ -706,7 +709,7 @@ int ensure_cube_fds(const LaunchPlan& lp, cx_exec_ctx* c, cudaStream_t s) {
 constexpr uint64_t kCubeMaxCells = 1ULL << 24;
 constexpr uint64_t kCubeMaxGlobalBytes = 8ULL << 30;
 constexpr uint64_t kCubeSmemBudget = 96 * 1024;
-constexpr uint64_t kCubeCellsPerChunk = 16384;
+constexpr uint64_t kCubeCellsPerChunk = 2048;
 constexpr uint64_t kDimSmemBudget = 96 * 1024;
 constexpr int64_t kDimGlobalKeys = 1LL << 26;  // keys of a dimension whose words may live in global memory
 
@@ -781,7 +784,9 @@ bool plan_cubes(const LaunchPlan& lp, const cx_exec_ctx* c, const int* shapes, i
     cp.cells[s] = cells;
     if (!used[s]) continue;
     cp.goff[s] = g;
-    g = align256(g + cells * (uint64_t)(sh.nsums + 1) * 8);
+    // Sums, then row counts or (no COUNT aggregate) presence bits.
+    const bool counts = lp.sshapes[s].naggs > sh.nsums;
+    g = align256(g + cells * (uint64_t)sh.nsums * 8 + (counts ? cells * 8 : (cells + 63) / 64 * 8));
     maxcells = std::max(maxcells, cells);
   }
   if (g > std::min(kCubeMaxGlobalBytes, c->cube_cap)) { cp.why = "the batch's cubes exceed the context's cube budget"; return false; }
@@ -852,6 +857,22 @@ bool plan_cubes(const LaunchPlan& lp, const cx_exec_ctx* c, const int* shapes, i
     dbytes += cd.first;
   }
   cp.dsm_bytes = dbytes;
+  // Presence bits of the global cubes without COUNT in what shared memory the
+  // scan's residency leaves, smallest cube first.
+  cp.pres_off.assign(nshapes, -1);
+  size_t ki = 0;
+  while (ki < lp.kernels.size() && lp.kernels[ki].kind != "cubescan") ++ki;
+  if (ki < lp.kernels.size()) {
+    const uint64_t taken = lp.kernels[ki].smem + cp.dsm_bytes + cp.smem_words * 8;
+    const uint64_t room = 227 * 1024 / (uint64_t)std::max(1, lp.kernels[ki].ctas_per_sm) - 1024;
+    for (int s : order) {
+      if (cp.smem_off[s] >= 0 || lp.sshapes[s].naggs > lp.cshapes[s].nsums) continue;
+      const uint64_t w = (cp.cells[s] + 31) / 32;
+      if (taken + (cp.pres_words + w) * 4 > room) continue;
+      cp.pres_off[s] = (int)cp.pres_words;
+      cp.pres_words += w;
+    }
+  }
   cp.on = true;
   return true;
 }
@@ -869,7 +890,9 @@ void fill_cube_args(CxArgs& a, const CubePlan& cp, int nshapes, char* scratch, u
     a.cube_g[s] = scratch && cp.used[s] && cp.cells[s] ? (unsigned long long*)(scratch + cube_off + cp.goff[s]) : nullptr;
     a.cube_cells[s] = (long long)cp.cells[s];
     a.cube_smem[s] = cp.smem_off[s];
+    a.cube_pres[s] = cp.pres_off[s];
   }
+  a.cube_pres_words = (int)cp.pres_words;
   a.cube_smem_words = (int)cp.smem_words;
   a.cube_chunks = cp.chunks;
   for (int d = 0; d < CX_MAX_HTS; ++d) {
@@ -1714,7 +1737,7 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
     P.qn = qn;
     P.nparams = poff;
     P.hstage = hstage;
-    P.extra_smem = cube ? (size_t)cp.dsm_bytes + (size_t)cp.smem_words * 8 : qb_bytes + (size_t)tab_words * 8 + (size_t)bit_words * 4 + 16;
+    P.extra_smem = cube ? (size_t)cp.dsm_bytes + (size_t)cp.smem_words * 8 + (size_t)cp.pres_words * 4 : qb_bytes + (size_t)tab_words * 8 + (size_t)bit_words * 4 + 16;
     P.scan_fn = L->fns[scan_ki];
     if (cube) {
       CUfunction spec = nullptr;
