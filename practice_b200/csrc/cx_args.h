@@ -96,6 +96,8 @@ struct CxArgs {
   // shape the u32 offset of its bits in shared memory (-1: in the cube itself).
   int cube_pres[CX_MAX_SHAPES];
   int cube_pres_words;                         // u32 words of all of them
-  unsigned char* zero_base;                    // plain queries: the scratch an execute starts from zeroed
+  unsigned char* zero_base;                    // the scratch that an execute or a shared pass starts from zeroed
   long long zero_bytes;
+  int zero_parts;                              // shared passes: blocks per query of the zeroing and key kernels
+  int zero_err;                                // 1: the zeroing kernel clears the error word too
 };

@@ -2428,38 +2428,61 @@ struct SharedGen {
   // Per pass: zeroes every query's result words, validity words and touched
   // bits (one block per query), so a pass has the same launches whatever its
   // queries' buffers are.
+  // What a pass starts from, in one launch: each query's result and validity
+  // words (zero_parts blocks a query), then the scratch -- dimension entries,
+  // touched bits, aggregate cubes -- and before the first pass the error word.
+  // One block per query took 10 us for 28,000 words and 30 ms for a 330 MB
+  // result, and the scratch was two memsets more.
   void emit_zero() {
-    meta << "kernel shared_zero zero 0 256 0\n";
+    meta << "kernel shared_zero zeroall 0 256\n";
     src << "extern \"C\" __global__ void __launch_bounds__(256) shared_zero(const CxArgs a) {\n";
-    src << "  const int q = blockIdx.x;\n";
-    src << "  if (q >= a.sq_total) return;\n";
+    src << "  const int cx_parts = a.zero_parts;\n";
+    src << "  const long long q = blockIdx.x / cx_parts;\n";
+    src << "  if (a.zero_err && blockIdx.x == 0 && threadIdx.x == 0) *a.err = 0u;\n";
+    src << "  if (q >= a.sq_total) {\n";
+    src << "    const long long cx_first = (long long)a.sq_total * cx_parts;\n";
+    src << "    for (long long i = (blockIdx.x - cx_first) * 256 + threadIdx.x; i < a.zero_bytes / 16; i += (gridDim.x - cx_first) * 256)\n";
+    src << "      ((uint4*)a.zero_base)[i] = make_uint4(0u, 0u, 0u, 0u);\n";
+    src << "    return;\n";
+    src << "  }\n";
     src << "  const CxSQ Q = a.sq[q];\n";
-    src << "  long long nw = 0, nt = 0;\n";
+    src << "  if (Q.keep) return;  // a query continuing over a later row range keeps its result\n";
+    src << "  long long nw = 0;\n";
     src << "  switch (Q.shape) {\n";
     for (size_t si = 0; si < shapes.size(); ++si) {
-      const Plan& p = *shapes[si];
-      Emitter e(p, tu);
-      const unsigned long long G = e.total_groups();
-      src << "    case " << si << ": nw = " << G * (unsigned long long)p.storage_ts() << "LL; nt = "
-          << (p.groups.empty() ? 0ULL : (G + 31) / 32) << "LL; break;\n";
+      Emitter e(*shapes[si], tu);
+      src << "    case " << si << ": nw = " << e.total_groups() * (unsigned long long)shapes[si]->storage_ts() << "LL; break;\n";
     }
     src << "    default: break;\n";
     src << "  }\n";
-    src << "  const long long nv = (nw + 63) / 64;\n";
-    src << "  if (!Q.keep) {  // a query continuing over a later row range keeps its result\n";
-    src << "    for (long long i = threadIdx.x; i < nw; i += blockDim.x) Q.result[i] = 0ULL;\n";
-    src << "    for (long long i = threadIdx.x; i < nv; i += blockDim.x) Q.validity[i] = 0ULL;\n";
-    src << "  }\n";
-    src << "  if (Q.touched)\n";
-    src << "    for (long long i = threadIdx.x; i < nt; i += blockDim.x) Q.touched[i] = 0u;\n";
+    src << "  const long long cx_i = (long long)(blockIdx.x % cx_parts) * 256 + threadIdx.x, cx_n = (long long)cx_parts * 256;\n";
+    src << "  for (long long i = cx_i; i < nw; i += cx_n) Q.result[i] = 0ULL;\n";
+    src << "  for (long long i = cx_i; i < (nw + 63) / 64; i += cx_n) Q.validity[i] = 0ULL;\n";
+    src << "}\n\n";
+  }
+
+  // The dimension indexes of one path in one launch: `parts` are device
+  // functions over a block number and count of their own (a block per 256
+  // rows; one after another, four of these kernels took 20 us of a small batch).
+  void emit_index_kernel(const char* kname, const char* kind, const std::vector<std::pair<std::string, int>>& parts) {
+    if (parts.empty()) return;
+    meta << "kernel " << kname << " " << kind << " 0 256 256 " << 148 * 16 << " " << parts.size();
+    for (const auto& pt : parts) meta << " " << pt.second;
+    meta << "\n";
+    src << "extern \"C\" __global__ void __launch_bounds__(256) " << kname << "(const CxArgs a) {\n";
+    src << "  long long cx_b = blockIdx.x;\n";
+    for (const auto& pt : parts) {
+      src << "  { const long long cx_n = cx::build_blocks(a.rows[" << pt.second << "], 256, " << 148 * 16 << ");\n";
+      src << "    if (cx_b < cx_n) { " << pt.first << "(a, cx_b, cx_n); return; }\n";
+      src << "    cx_b -= cx_n; }\n";
+    }
     src << "}\n\n";
   }
 
   // Per batch: slot entries of one dimension with the batch's query masks.
-  void emit_index(const Dim& d, int di) {
+  std::string emit_index(const Dim& d, int di) {
     const std::string k = "index_" + lower(d.name);
-    meta << "kernel " << k << " build " << d.table << " 256 1024\n";
-    src << "extern \"C\" __global__ void __launch_bounds__(256) " << k << "(const CxArgs a) {\n";
+    src << "__device__ __forceinline__ void " << k << "(const CxArgs& a, long long cx_block, long long cx_blocks) {\n";
     src << "  __shared__ int s_shape[" << MAXQ << "], s_poff[" << MAXQ << "];\n";
     src << "  const int nq = a.sq_total < " << MAXQ << " ? a.sq_total : " << MAXQ << ";\n";
     src << "  for (int q = threadIdx.x; q < nq; q += blockDim.x) { s_shape[q] = a.sq[q].shape; s_poff[q] = a.sq[q].param_off; }\n";
@@ -2471,7 +2494,7 @@ struct SharedGen {
     for (size_t i = 0; i < d.attrs.size(); ++i)
       src << "  const int* __restrict__ at" << i << " = a.col[" << slot_of(d.attrs[i], d.table) << "];\n";
     for (const auto& c : d.fcols) src << "  const int* __restrict__ F_" << c << " = a.col[" << slot_of(c, d.table) << "];\n";
-    src << "  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {\n";
+    src << "  for (long long r = cx_block * 256 + threadIdx.x; r < n; r += cx_blocks * 256) {\n";
     src << "    const int k = key[r];\n";
     src << "    if (k == 0) continue;\n";
     src << "    const int h = (int)HASH(k, " << d.len << ", " << d.keymin << ");\n";
@@ -2503,6 +2526,7 @@ struct SharedGen {
       src << ", 0);\n";
     }
     src << "  }\n}\n\n";
+    return k;
   }
 
   // ------------------------------------------------------ aggregate cubes --
@@ -2600,11 +2624,10 @@ struct SharedGen {
   // whose queries its join filter passes (shapes that do not join the
   // dimension always set), and its cube attributes as 16-bit offsets from the
   // registered range minimum.
-  void emit_cube_index(const Dim& d, int di) {
+  std::string emit_cube_index(const Dim& d, int di) {
     const std::string k = "cube_index_" + lower(d.name);
-    meta << "kernel " << k << " cubeidx " << d.table << " 256 1024\n";
     std::ostringstream& o = src;
-    o << "extern \"C\" __global__ void __launch_bounds__(256) " << k << "(const CxArgs a) {\n";
+    o << "__device__ __forceinline__ void " << k << "(const CxArgs& a, long long cx_block, long long cx_blocks) {\n";
     o << "  const long long n = a.rows[" << d.table << "];\n";
     o << "  int4* ent = (int4*)a.ht[" << d.slot << "];\n";
     o << "  const int* __restrict__ key = a.col[" << slot_of(d.pk, d.table) << "];\n";
@@ -2618,7 +2641,7 @@ struct SharedGen {
     unsigned nj = 0;
     for (size_t s = 0; s < shapes.size(); ++s)
       if (!preds[s].joins.count(di)) nj |= 1u << s;
-    o << "  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {\n";
+    o << "  for (long long r = cx_block * 256 + threadIdx.x; r < n; r += cx_blocks * 256) {\n";
     o << "    const int k = key[r];\n";
     o << "    if (k == 0) continue;\n";
     o << "    const int h = (int)HASH(k, " << d.len << ", " << d.keymin << ");\n";
@@ -2668,6 +2691,7 @@ struct SharedGen {
     o << "    if (atomicCAS(&ent[h].x, 0, k) != 0) { cx::raise(a.err, cx::ERR_DIM_COLLISION); continue; }\n";
     o << "    ent[h] = make_int4(k, (int)rel, (int)(f_[0] | (f_[1] << 16)), (int)(f_[2] | (f_[3] << 16)));\n";
     o << "  }\n}\n\n";
+    return k;
   }
 
   // One pass over the fact rows: warp tiles of 32 x IPT rows read with vector
@@ -3163,7 +3187,7 @@ struct SharedGen {
     collect();
     if (tu.cube > 0) collect_cube();
     else cube_why = "cube path switched off";
-    meta << "v 1\nshared " << MAXQ << " " << MAXQ * std::max(1, max_lits) << "\n";
+    meta << "v 2\nshared " << MAXQ << " " << MAXQ * std::max(1, max_lits) << "\n";
     for (const Dim& d : dims) {
       meta << "ht " << d.slot << " dkm_" << lower(d.name) << " " << d.len * 4 << "\n";
       if (d.attrs.size() > 1) meta << "dat " << d.slot << " " << d.len * 4 << "\n";
@@ -3195,9 +3219,14 @@ struct SharedGen {
              << dims[di].fk << " d_" << dims[di].pk << "\n";
     }
     emit_zero();
-    for (size_t di = 0; di < dims.size(); ++di) emit_index(dims[di], (int)di);
-    if (cube_why.empty())
-      for (size_t di = 0; di < dims.size(); ++di) emit_cube_index(dims[di], (int)di);
+    std::vector<std::pair<std::string, int>> parts;
+    for (size_t di = 0; di < dims.size(); ++di) parts.emplace_back(emit_index(dims[di], (int)di), dims[di].table);
+    emit_index_kernel("index_tables", "builds", parts);
+    if (cube_why.empty()) {
+      parts.clear();
+      for (size_t di = 0; di < dims.size(); ++di) parts.emplace_back(emit_cube_index(dims[di], (int)di), dims[di].table);
+      emit_index_kernel("cube_index_tables", "cubebuilds", parts);
+    }
     emit_scan();
     if (cube_why.empty()) {
       emit_cube_scan();
@@ -4004,9 +4033,9 @@ struct SharedGen {
   }
 
   void emit_keys() {
-    meta << "kernel shared_keys_epilogue queries 0 256 0\n";
+    meta << "kernel shared_keys_epilogue queryparts 0 256\n";
     src << "extern \"C\" __global__ void __launch_bounds__(256) shared_keys_epilogue(const CxArgs a) {\n";
-    src << "  const int q = blockIdx.x;\n";
+    src << "  const int q = blockIdx.x / a.zero_parts;\n";
     src << "  if (q >= a.sq_total) return;\n";
     src << "  const CxSQ Q = a.sq[q];\n";
     src << "  unsigned long long* d_result = Q.result; (void)d_result;\n";
@@ -4017,7 +4046,8 @@ struct SharedGen {
       if (p.groups.empty()) continue;
       Emitter e(p, tu);
       src << "    case " << s << ":\n";
-      src << "      for (long long g = threadIdx.x; g < " << e.total_groups() << "LL; g += blockDim.x) {\n";
+      src << "      for (long long g = (long long)(blockIdx.x % a.zero_parts) * 256 + threadIdx.x; g < " << e.total_groups()
+          << "LL; g += (long long)a.zero_parts * 256) {\n";
       src << "        if (!((Q.touched[g >> 5] >> (g & 31)) & 1u)) continue;\n";
       e.emit_key_store(src, "g", "        ");
       src << "      }\n      break;\n";

@@ -110,6 +110,7 @@ struct KernelSpec {
 };
 
 struct LaunchPlan {
+  int version = 1;
   std::vector<std::string> tables;
   struct Col { int slot; std::string name; int table; };
   std::vector<Col> cols;
@@ -166,7 +167,9 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
     if (k == "v") {
       int v = 0;
       ls >> v;
-      if (v != 1) { err = "unsupported launch plan version"; return false; }
+      // 2: shared programs whose cubes without COUNT end in presence bits (1: in words).
+      if (v != 1 && v != 2) { err = "unsupported launch plan version"; return false; }
+      lp.version = v;
     } else if (k == "table") {
       int s; std::string n;
       ls >> s >> n;
@@ -275,7 +278,7 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
       KernelSpec ks;
       ls >> ks.name >> ks.kind >> ks.table >> ks.block;
       if (ks.kind == "build" || ks.kind == "cubeidx" || ks.kind == "tiles" || ks.kind == "tilescan") ls >> ks.tile;
-      else if (ks.kind == "builds") {
+      else if (ks.kind == "builds" || ks.kind == "cubebuilds") {
         size_t n = 0;
         ls >> ks.tile >> ks.cap >> n;
         for (size_t i = 0; i < n && ls; ++i) {
@@ -283,7 +286,7 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
           ls >> t;
           ks.parts.push_back(t);
         }
-      } else if (ks.kind == "prep") {
+      } else if (ks.kind == "prep" || ks.kind == "zeroall" || ks.kind == "queryparts") {
       } else if (ks.kind == "scan" || ks.kind == "sharedscan" || ks.kind == "cubescan") ls >> ks.tile >> ks.smem >> ks.ctas_per_sm;
       else { size_t z; ls >> z; }
       lp.kernels.push_back(ks);
@@ -309,7 +312,7 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
       return false;
     }
   for (const auto& k : lp.kernels) {
-    if (k.kind != "builds") continue;
+    if (k.kind != "builds" && k.kind != "cubebuilds") continue;
     bool ok = k.tile > 0 && k.block > 0 && k.block <= 1024 && k.cap > 0 && !k.parts.empty();
     for (int t : k.parts) ok = ok && t >= 0 && t < (int)lp.tables.size();
     if (!ok) {
@@ -785,7 +788,7 @@ bool plan_cubes(const LaunchPlan& lp, const cx_exec_ctx* c, const int* shapes, i
     if (!used[s]) continue;
     cp.goff[s] = g;
     // Sums, then row counts or (no COUNT aggregate) presence bits.
-    const bool counts = lp.sshapes[s].naggs > sh.nsums;
+    const bool counts = lp.sshapes[s].naggs > sh.nsums || lp.version < 2;
     g = align256(g + cells * (uint64_t)sh.nsums * 8 + (counts ? cells * 8 : (cells + 63) / 64 * 8));
     maxcells = std::max(maxcells, cells);
   }
@@ -862,7 +865,7 @@ bool plan_cubes(const LaunchPlan& lp, const cx_exec_ctx* c, const int* shapes, i
   cp.pres_off.assign(nshapes, -1);
   size_t ki = 0;
   while (ki < lp.kernels.size() && lp.kernels[ki].kind != "cubescan") ++ki;
-  if (ki < lp.kernels.size()) {
+  if (ki < lp.kernels.size() && lp.version >= 2) {
     const uint64_t taken = lp.kernels[ki].smem + cp.dsm_bytes + cp.smem_words * 8;
     const uint64_t room = 227 * 1024 / (uint64_t)std::max(1, lp.kernels[ki].ctas_per_sm) - 1024;
     for (int s : order) {
@@ -1663,6 +1666,15 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
     c->host_stage_bytes = stage_bytes * 2;
   }
 
+  // Blocks per query of the zeroing and key kernels: one per 2048 result words
+  // of the largest query, so that a large result is not left to one block.
+  uint64_t most_words = 1;
+  for (int i = 0; i < nq; ++i) most_words = std::max(most_words, lp.sshapes[queries[i].shape].groups * (uint64_t)lp.sshapes[queries[i].shape].ts);
+  a.zero_base = (unsigned char*)scratch;
+  a.zero_bytes = (long long)(cube ? cube_off + cp.gbytes : touch_end);
+  a.zero_parts = (int)std::min<uint64_t>(256, (most_words + 2047) / 2048);
+  const bool zero_all = !lp.kernels.empty() && lp.kernels[0].kind == "zeroall";
+
   size_t scan_ki = 0;
   const char* scan_kind = cube ? "cubescan" : "sharedscan";
   while (scan_ki < lp.kernels.size() && lp.kernels[scan_ki].kind != scan_kind) ++scan_ki;
@@ -1733,6 +1745,7 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
       if (s < CX_MAX_SHAPES) { if (a.sq_num[s] == 0) a.sq_first[s] = j; ++a.sq_num[s]; }
     }
     if (cube) fill_cube_args(a, cp, nshapes, scratch, cube_off);
+    a.zero_err = ps == 0 ? 1 : 0;
     P.args = a;
     P.qn = qn;
     P.nparams = poff;
@@ -1773,20 +1786,30 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
       return CX_OK;
     };
     CX_CUDA(rec(c->ev[0]));
-    CX_CUDA(cudaMemsetAsync(scratch + err_off, 0, 16, s));
+    if (!zero_all || npass == 0) CX_CUDA(cudaMemsetAsync(scratch + err_off, 0, 16, s));
     for (int ps = 0; ps < npass; ++ps) {
       Pass& P = passes[ps];
-      CX_CUDA(cudaMemcpyAsync((void*)P.args.sq, P.hstage, (size_t)P.qn * sizeof(CxSQ), cudaMemcpyHostToDevice, s));
-      if (P.nparams)
+      // Descriptors and parameters: one copy where they lie side by side.
+      const bool joined = P.qn == maxq;
+      CX_CUDA(cudaMemcpyAsync((void*)P.args.sq, P.hstage, joined ? desc_bytes + (size_t)P.nparams * 4 : (size_t)P.qn * sizeof(CxSQ),
+                              cudaMemcpyHostToDevice, s));
+      if (P.nparams && !joined)
         CX_CUDA(cudaMemcpyAsync((void*)P.args.sparams, P.hstage + desc_bytes, (size_t)P.nparams * 4, cudaMemcpyHostToDevice, s));
-      CX_CUDA(cudaMemsetAsync(scratch, 0, dim_end, s));
-      if (cube && cp.gbytes) CX_CUDA(cudaMemsetAsync(scratch + cube_off, 0, cp.gbytes, s));
+      if (!zero_all) {
+        CX_CUDA(cudaMemsetAsync(scratch, 0, dim_end, s));
+        if (cube && cp.gbytes) CX_CUDA(cudaMemsetAsync(scratch + cube_off, 0, cp.gbytes, s));
+      }
       // Before the scan: result zeroing and the path's dimension indexes; after
       // it: the cube answers (cube path) and the group-key epilogue.
       for (size_t ki = 0; ki < scan_ki; ++ki) {
         const KernelSpec& k = lp.kernels[ki];
-        unsigned grid;
-        if (k.kind == "zero") grid = (unsigned)P.qn;
+        unsigned grid = 0;
+        if (k.kind == "zeroall")
+          grid = (unsigned)((uint64_t)P.qn * P.args.zero_parts +
+                            std::min<uint64_t>(((uint64_t)P.args.zero_bytes / 16 + k.block - 1) / k.block, (uint64_t)sms * 8));
+        else if (k.kind == "zero") grid = (unsigned)P.qn;
+        else if (k.kind == (cube ? "cubebuilds" : "builds"))
+          for (int t : k.parts) grid += (unsigned)std::min<long long>((rows[t] + k.tile - 1) / k.tile, k.cap);
         else if (k.kind == (cube ? "cubeidx" : "build"))
           grid = (unsigned)std::min<long long>((rows[k.table] + k.tile - 1) / k.tile, (long long)sms * 16);
         else continue;
@@ -1801,6 +1824,7 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
         const KernelSpec& k = lp.kernels[ki];
         unsigned grid;
         if (k.kind == "queries") grid = (unsigned)P.qn;
+        else if (k.kind == "queryparts") grid = (unsigned)P.qn * (unsigned)P.args.zero_parts;
         else if (cube && k.kind == "cubeans") grid = (unsigned)(P.qn * cp.chunks);
         else continue;
         if ((r = launch(ki, grid, 0, &P.args))) return r;
