@@ -930,7 +930,7 @@ CX_DEVICE long long build_blocks(long long rows, int tile, int cap) {
 }
 
 // ProbeMultiHT over the generated build's directory of four ints per slot
-// (key, offset, count, and the build's write cursor): one 16-byte load.
+// (key, offset, count, first published value): one 16-byte load.
 CX_DEVICE void ProbeMultiHT4(int key, int& offset, int& count, int& flag, const int* ht_dir, int ht_len, int key_min) {
   count = 0;
   if (!flag) return;
