@@ -3225,7 +3225,6 @@ struct SharedGen {
             o << "        { const unsigned long long v_ = cg_[" << ks << "ULL * (unsigned long long)nc_ + c]; if (v_) atomicAdd(&d_result[" << ix << "], v_); }\n";
             ++ks;
           }
-          if (!p.sparse) o << "        db::atomic_set_valid_bit(d_result_validity, " << ix << ");\n";
         }
       }
       o << "      }\n";
@@ -3256,7 +3255,7 @@ struct SharedGen {
       const bool smem_ok = !p.groups.empty() && G * NA * 8 <= 4096ULL;
       meta << "sshape " << s << " " << G << " " << p.storage_ts() << " " << (p.groups.empty() ? 0 : 1)
            << " " << (p.sparse ? 1 : 0) << " " << lit_maps[s].size() << " " << (smem_ok ? 1 : 0) << " " << NA << " "
-           << (G + 31) / 32 << " " << nseen << "\n";
+           << (G + 31) / 32 << " " << nseen << " " << qtab_of(p).u64 << " " << qtab_of(p).bits << "\n";
     }
     if (cube_why.empty()) {
       meta << "cube " << cattrs.size() << "\n";
@@ -3301,112 +3300,103 @@ struct SharedGen {
     return out.str();
   }
 
-  // CTA-tiled shared scan.  Per tile of TR = block x items rows: thread 0
-  // stages the union of fact columns by TMA bulk copies; every thread builds
-  // the query masks of its rows (filter tables, one gather per dimension,
-  // residual filters) and stores them with the payload attributes in shared
-  // memory; then warps take (query, row slice) units and aggregate the rows
-  // whose mask bit is set.
-  void emit_scan() {
-    const int CTA = tu.block_threads, IPT = tu.items_per_thread;
-    if (CTA % 32 || CTA < 64 || CTA > 1024 || IPT < 1 || IPT > 16) throw PlanError("bad block shape");
-    const int NW = CTA / 32, TR = CTA * IPT;
-    if (NW < 3) throw PlanError("shared scan needs at least 3 warps (staging, masks, aggregation)");
-    // Warp roles: warp 0 stages tiles, NPW warps build masks, the rest aggregate.
-    const int NPW = tu.producer_warps > 0 ? std::min(tu.producer_warps, NW - 2) : std::max(1, (NW - 1) * 3 / 8);
-    const int NCW = NW - 1 - NPW;
-    const int NSC = (int)fact_cols.size();
-    int STAGES = std::max(2, tu.stages);
-    const int MAXP = MAXQ * std::max(1, max_lits);
-    const int NACC = std::max(1, max_scalar_aggs) * 2;  // (sum, count) per scalar aggregate
-    const int NFC = (int)fcols.size();
-    int nattr = 0;
-    std::map<std::string, int> attr_slot;
-    for (const Dim& d : dims)
-      for (const auto& at : d.attrs) attr_slot[at] = nattr++;
-    // Shapes with a small group domain and literal-free group keys get per-group
-    // row bitmaps (plus one word of out-of-domain rows) built with the masks.
-    std::vector<int> gm_base(shapes.size(), -1);
-    int gm_words = 0;
-    for (size_t si = 0; si < shapes.size(); ++si) {
-      const Plan& p = *shapes[si];
-      if (p.groups.empty() || tu.group_merge == 2) continue;
-      Emitter e(p, tu);
-      const unsigned long long G = e.total_groups();
-      std::vector<const Expr*> gl;
-      for (const auto& g : p.groups) lits_of(g.expr.get(), gl);
-      if (G <= 31 && G * p.aggs.size() <= 16 && gl.empty()) {
-        gm_base[si] = gm_words;
-        gm_words += (int)G + 1;
-      }
+  // Words of one group in a query's shared-memory table (a SUM is a low and a
+  // high 32-bit word, a COUNT one word), the copies of each word (lane modulo
+  // copies, so that lanes on one group hit different banks: 32 for a scalar or a
+  // few groups) and the table's bytes; a table of more than 4 KB per query is not
+  // kept (its rows go to the result with global atomics).
+  struct QTab { int words = 0, rep = 1; unsigned long long u64 = 0, bits = 0; bool counts = false; };
+  QTab qtab_of(const Plan& p) const {
+    QTab t;
+    Emitter e(p, tu);
+    const unsigned long long G = e.total_groups();
+    for (const auto& ag : p.aggs) {
+      t.words += ag.fn == AggFn::Count ? 1 : 2;
+      t.counts = t.counts || ag.fn == AggFn::Count;
     }
-    // Fewer stages when the ring would not leave room for the rest.
-    while (STAGES > 2 && (unsigned long long)STAGES * ((unsigned long long)(NSC + nattr) * TR * 4 + (MAXQ + gm_words) * (TR / 32) * 4) > 160 * 1024) --STAGES;
-    unsigned long long off = 0;
-    const int NB = TR / 32;  // 32-row blocks per tile
-    // Row stride of a query's (or a group's) block words: one word of padding,
-    // so the 32 lanes of a mask warp, each storing the word of its own query
-    // for the same block, hit 32 different banks.
-    const int NBS = NB + 1;
-    // Per stage: the fact columns, the payload attributes and the per-query row bitmaps of one tile.
-    const unsigned long long stage_off = off; off += (unsigned long long)STAGES * NSC * TR * 4;
-    const unsigned long long attr_off = off; off += (unsigned long long)STAGES * nattr * TR * 4;
-    const unsigned long long gm_off = off; off += (unsigned long long)STAGES * gm_words * NBS * 4;
-    const unsigned long long bars_off = off; off += (unsigned long long)STAGES * 3 * 8 + 16;
-    off = (off + 15) & ~15ULL;
+    const unsigned long long one = G * t.words * 4;
+    if (one > 4096) return t;
+    while (t.rep < 32 && one * t.rep * 2 <= 4096) t.rep *= 2;
+    t.u64 = (one * t.rep + 7) / 8;
+    t.bits = t.counts ? 0 : (G + 31) / 32;
+    return t;
+  }
+
+  // Shared scan by per-query row masks.  Every warp walks tiles of 32 x IPT
+  // rows: per row the mask of the queries that keep it (filter tables, then one
+  // gather per dimension, small dimensions first so that rows no query joins
+  // skip the large ones, then residual filters), and per shape with bits left
+  // the group and the aggregate values once, then one update per set bit into
+  // that query's table.  Rows stay in the registers of one warp: with masks
+  // handed from mask warps to aggregation warps through shared memory (row
+  // bitmaps per query, transposed, walked bit by bit) a 32-query batch took
+  // 798 warp instructions per 32 rows, most of them for the hand-over.
+  // Measured at 60M rows, scan: 8 / 16 / 32 / 64 mixed queries 1.77 / 1.83 /
+  // 2.05 / 3.27 -> 1.00 / 1.19 / 1.47 / 2.23 ms; bound by the L1 pipe (a 16-byte
+  // gather per joined dimension and row, each lane its own line) and issue.
+  void emit_scan() {
+    const int CTA = tu.block_threads;
+    if (CTA % 32 || CTA < 64 || CTA > 1024 || tu.items_per_thread < 1 || tu.items_per_thread > 16) throw PlanError("bad block shape");
+    if (CTA / 32 < 3) throw PlanError("shared scan needs at least 3 warps");
+    const int IPT = 2, VW = 2, NW = CTA / 32;
+    const int MAXP = MAXQ * std::max(1, max_lits);
+    const int NFC = (int)fcols.size(), ND = (int)dims.size(), NSH = (int)shapes.size();
+    const size_t NSC = fact_cols.size();
+    if (NSC > 64) throw PlanError("more than 64 fact columns in a shared batch");
+    unsigned long long off = 16;
     const unsigned long long par_off = off; off += (unsigned long long)MAXP * 4;
     off = (off + 15) & ~15ULL;
-    const unsigned long long acc_off = off; off += (unsigned long long)MAXQ * NACC * 8;
     const unsigned long long sq_off = off; off += ((unsigned long long)MAXQ * sizeof(CxSQ) + 15) & ~15ULL;
+    const unsigned long long qt_off = off; off += (unsigned long long)MAXQ * 8;  // per query: table and bit offsets
     const unsigned long long fm_off = off; off += (unsigned long long)NFC * FW * 8;
-    const unsigned long long nj_off = off; off += (unsigned long long)(dims.size() + 4) * 8;
-    off = (off + 15) & ~15ULL;
-    // The per-query row bitmaps (STAGES x NB words per query of the pass) and
-    // the group tables follow the fixed part; the host sizes both per pass.
-    const unsigned long long qb_off = (off + 15) & ~15ULL;
-    const unsigned long long smem_total = qb_off;
-    if (smem_total + (unsigned long long)MAXQ * STAGES * NBS * 4 > 200 * 1024)
-      throw PlanError("shared scan shared memory exceeds 200 KB before group tables");
-    meta << "sqb " << STAGES * NBS * 4 << "\n";
+    const unsigned long long nj_off = off; off += (unsigned long long)(ND + 4) * 8;
+    const unsigned long long tab_off = (off + 15) & ~15ULL;
     const unsigned wait_limit = (unsigned)std::min(60000000, std::max(1, tu.wait_limit_us));
     const std::string kname = "SharedScan_" + fact;
-    meta << "kernel " << kname << " sharedscan 0 " << CTA << " " << TR << " " << smem_total << " " << tu.ctas_per_sm << "\n";
+    meta << "kernel " << kname << " sharedscan 0 " << CTA << " " << 32 * IPT * NW << " " << tab_off << " " << tu.ctas_per_sm << "\n";
 
     std::ostringstream& o = src;
     // At least 32 resident warps per SM: registers are capped at 64.
     o << "extern \"C\" __global__ void __launch_bounds__(" << CTA << ", " << std::max(1, 1024 / CTA) << ") " << kname << "(const CxArgs a) {\n";
-    o << "  constexpr int TR = " << TR << ", NSTAGE = " << STAGES << ", NSC = " << NSC << ", NPW = " << NPW << ", NCW = " << NCW << ";\n";
-    o << "  extern __shared__ __align__(1024) unsigned char cx_smem[];\n";
+    o << "  constexpr int IPT = " << IPT << ", VW = " << VW << ", TROWS = " << 32 * IPT << ";\n";
+    o << "  extern __shared__ __align__(16) unsigned char cx_smem[];\n";
     if (tu.debug_stall)
       o << "  { cx::debug_stall((unsigned long long*)cx_smem, a.err, " << wait_limit << "u); return; }\n";
     o << "  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;\n";
-    o << "  int* stage_buf = (int*)(cx_smem + " << stage_off << ");\n";
-    o << "  int* s_attr = (int*)(cx_smem + " << attr_off << "); (void)s_attr;\n";
-    o << "  unsigned* s_qb = (unsigned*)(cx_smem + " << qb_off << ");  // [stage][query][32-row block] row bitmaps\n";
-    o << "  const int nq_ = a.sq_total < " << MAXQ << " ? a.sq_total : " << MAXQ << ";\n";
-    o << "  unsigned* s_gm = (unsigned*)(cx_smem + " << gm_off << "); (void)s_gm;  // [stage][shape group][32-row block]\n";
-    o << "  unsigned long long* bar_full = (unsigned long long*)(cx_smem + " << bars_off << ");   // tile staged\n";
-    o << "  unsigned long long* bar_ready = bar_full + NSTAGE;   // masks built\n";
-    o << "  unsigned long long* bar_empty = bar_full + 2 * NSTAGE;  // aggregation done\n";
-    o << "  volatile int* s_abort = (volatile int*)(bar_full + 3 * NSTAGE);\n";
-    o << "  int* s_nissued = (int*)(bar_full + 3 * NSTAGE) + 1;\n";
     o << "  int* s_params = (int*)(cx_smem + " << par_off << ");\n";
-    o << "  unsigned long long* s_qacc = (unsigned long long*)(cx_smem + " << acc_off << ");\n";
     o << "  CxSQ* s_sq = (CxSQ*)(cx_smem + " << sq_off << ");\n";
+    o << "  int2* s_qt = (int2*)(cx_smem + " << qt_off << ");  // u32 offsets of a query's table (-1: none) and presence bits\n";
     o << "  unsigned long long* s_fm = (unsigned long long*)(cx_smem + " << fm_off << "); (void)s_fm;\n";
     o << "  unsigned long long* s_nj = (unsigned long long*)(cx_smem + " << nj_off << ");\n";
-    o << "  unsigned long long* s_tab = (unsigned long long*)(cx_smem + " << qb_off << " + ((NSTAGE * nq_ * " << NBS * 4 << " + 15) & ~15)); (void)s_tab;\n";
-    o << "  unsigned int* s_bits = (unsigned int*)(s_tab + a.smem_tab_words); (void)s_bits;\n";
+    o << "  unsigned* s_tab = (unsigned*)(cx_smem + " << tab_off << ");\n";
+    o << "  unsigned* s_bits = s_tab + 2 * a.smem_tab_words;\n";
     o << "  const int nq = a.sq_total < " << MAXQ << " ? a.sq_total : " << MAXQ << ";\n";
-    o << "  const long long n_rows = a.rows[0];\n";
-    o << "  const long long num_tiles = (n_rows + TR - 1) / TR;\n";
-    o << "  const long long full_tiles = n_rows / TR;\n";
-    o << "  for (int w = threadIdx.x; w < nq; w += " << CTA << ") s_sq[w] = a.sq[w];\n";
-    o << "  for (int w = threadIdx.x; w < a.nparams && w < " << MAXP << "; w += " << CTA << ") s_params[w] = a.sparams[w];\n";
-    o << "  for (int w = threadIdx.x; w < " << MAXQ * NACC << "; w += " << CTA << ") s_qacc[w] = 0ULL;\n";
-    o << "  for (int w = threadIdx.x; w < a.smem_tab_words; w += " << CTA << ") s_tab[w] = 0ULL;\n";
-    o << "  for (int w = threadIdx.x; w < a.smem_bit_words; w += " << CTA << ") s_bits[w] = 0u;\n";
+    // Descriptors and parameters arrive by bulk copies (both 16-byte aligned,
+    // the parameters padded to 16 bytes) while the tables are cleared; the wait
+    // is bounded, and after it gives up the copies in flight are waited for.
+    const std::string LIM = std::to_string(wait_limit) + "u";
+    o << "  unsigned long long* bars = (unsigned long long*)cx_smem;\n";
+    o << "  static_assert(sizeof(CxSQ) % 16 == 0, \"bulk copies take 16-byte units\");\n";
+    o << "  if (threadIdx.x == 0) {\n";
+    o << "    const unsigned cx_pb = (unsigned)((a.nparams < " << MAXP << " ? a.nparams : " << MAXP << ") * 4 + 15) & ~15u;\n";
+    o << "    const unsigned long long l2_policy = cx::l2_evict_first_policy();\n";
+    o << "    cx::mbar_init(bars, 1);\n";
+    o << "    cx::fence_mbar_init();\n";
+    o << "    cx::mbar_expect_tx(bars, (unsigned)(nq * sizeof(CxSQ)) + cx_pb);\n";
+    o << "    if (nq) cx::bulk_g2s(s_sq, a.sq, (unsigned)(nq * sizeof(CxSQ)), bars, l2_policy);\n";
+    o << "    if (cx_pb) cx::bulk_g2s(s_params, a.sparams, cx_pb, bars, l2_policy);\n";
+    o << "  }\n";
+    o << "  for (int w = threadIdx.x; w < 2 * a.smem_tab_words + a.smem_bit_words; w += " << CTA << ") s_tab[w] = 0u;\n";
     o << "  __syncthreads();\n";
+    o << "  if (!__syncthreads_and(cx::mbar_wait_bounded(bars, 0u, " << LIM << "))) {\n";
+    o << "    if (threadIdx.x == 0) {\n";
+    o << "      cx::raise(a.err, cx::ERR_WAIT_TIMEOUT);\n";
+    o << "      (void)cx::mbar_wait_bounded(bars, 0u, cx::drain_limit_us(" << LIM << "));\n";
+    o << "    }\n";
+    o << "    return;\n";
+    o << "  }\n";
+    o << "  for (int w = threadIdx.x; w < nq; w += " << CTA << ")\n";
+    o << "    s_qt[w] = make_int2(s_sq[w].smem_acc >= 0 ? 2 * s_sq[w].smem_acc : -1, s_sq[w].smem_bits);\n";
     // Filter tables: bit q of s_fm[k * FW + v] clears when query q's conjuncts
     // on filter column k reject the value fbase[k] + v.
     if (NFC) {
@@ -3418,7 +3408,7 @@ struct SharedGen {
       o << "      const int* P = s_params + s_sq[q].param_off; (void)P;\n";
       o << "      bool pass = true;\n";
       o << "      switch (s_sq[q].shape) {\n";
-      for (size_t s = 0; s < shapes.size(); ++s) {
+      for (int s = 0; s < NSH; ++s) {
         if (preds[s].pushed.empty()) continue;
         Emitter e(*shapes[s], tu);
         e.lit_index = &lit_maps[s];
@@ -3437,37 +3427,31 @@ struct SharedGen {
       o << "    s_fm[v] = m;\n";
       o << "  }\n";
     }
-    // Fact columns each shape reads (bits over the staged columns).
-    if (NSC > 64) throw PlanError("more than 64 fact columns in a shared batch");
-    const std::vector<unsigned long long> colmask = shape_colmasks();
     // Masks of the queries that skip each dimension, that carry residual
     // filters, that have filter-table conjuncts, and of the whole batch; and
     // the fact columns the batch reads.
+    const std::vector<unsigned long long> colmask = shape_colmasks();
     {
-      std::vector<unsigned> joins(shapes.size(), 0u);
-      std::vector<int> has_res(shapes.size(), 0), has_push(shapes.size(), 0);
-      for (size_t s = 0; s < shapes.size(); ++s) {
-        for (const auto& kv : preds[s].joins) joins[s] |= 1u << kv.first;
-        has_res[s] = !preds[s].resid.empty();
-        has_push[s] = !preds[s].pushed.empty();
-      }
-      o << "  if (threadIdx.x < " << dims.size() + 4 << ") {\n";
+      o << "  if (threadIdx.x < " << ND + 4 << ") {\n";
       o << "    const int t_ = threadIdx.x;\n";
       o << "    unsigned long long m = 0ULL;\n";
       o << "    for (int q = 0; q < nq; ++q) {\n";
       o << "      unsigned j_ = 0u; int r_ = 0, p_ = 0; unsigned long long c_ = 0ULL;\n";
       o << "      switch (s_sq[q].shape) {\n";
-      for (size_t s = 0; s < shapes.size(); ++s)
-        o << "        case " << s << ": j_ = " << joins[s] << "u; r_ = " << has_res[s] << "; p_ = " << has_push[s]
+      for (int s = 0; s < NSH; ++s) {
+        unsigned joins = 0u;
+        for (const auto& kv : preds[s].joins) joins |= 1u << kv.first;
+        o << "        case " << s << ": j_ = " << joins << "u; r_ = " << !preds[s].resid.empty() << "; p_ = " << !preds[s].pushed.empty()
           << "; c_ = " << colmask[s] << "ULL; break;\n";
+      }
       o << "        default: break;\n";
       o << "      }\n";
       o << "      bool b_ = false;\n";
-      o << "      if (t_ < " << dims.size() << ") b_ = !((j_ >> t_) & 1u);\n";
-      o << "      else if (t_ == " << dims.size() << ") b_ = r_ != 0;\n";
-      o << "      else if (t_ == " << dims.size() + 1 << ") b_ = p_ != 0;\n";
+      o << "      if (t_ < " << ND << ") b_ = !((j_ >> t_) & 1u);\n";
+      o << "      else if (t_ == " << ND << ") b_ = r_ != 0;\n";
+      o << "      else if (t_ == " << ND + 1 << ") b_ = p_ != 0;\n";
       o << "      else b_ = true;\n";
-      o << "      if (t_ == " << dims.size() + 3 << ") m |= c_;\n";
+      o << "      if (t_ == " << ND + 3 << ") m |= c_;\n";
       o << "      else if (b_) m |= 1ULL << q;\n";
       o << "    }\n";
       o << "    s_nj[t_] = m;\n";
@@ -3479,610 +3463,259 @@ struct SharedGen {
       if (d.attrs.size() > 1) o << "  const int4* __restrict__ dat_" << lower(d.name) << " = (const int4*)a.dat[" << d.slot << "];\n";
     }
     for (int k = 0; k < NFC; ++k) o << "  const unsigned fb" << k << " = (unsigned)a.fbase[" << k << "], fw" << k << " = (unsigned)a.fwin[" << k << "];\n";
-    o << "  bool staged_ok = true;\n";
-    for (const auto& c : fact_cols) o << "  staged_ok = staged_ok && ((((unsigned long long)d_" << c << ") & 15ULL) == 0ULL);\n";
-    o << "  unsigned long long l2_policy = 0;\n";
-    o << "  if (threadIdx.x == 0) {\n";
-    o << "    for (int s = 0; s < NSTAGE; ++s) {\n";
-    o << "      cx::mbar_init(&bar_full[s], 1);\n";
-    o << "      cx::mbar_init(&bar_ready[s], NPW);\n";
-    o << "      cx::mbar_init(&bar_empty[s], NCW);\n";
-    o << "    }\n";
-    o << "    *s_abort = 0;\n";
-    o << "    *s_nissued = 0;\n";
-    o << "    cx::fence_mbar_init();\n";
-    o << "    l2_policy = cx::l2_evict_first_policy();\n";
-    o << "  }\n";
-    // Only the columns the batch's shapes read are staged.
-    o << "#define CX_ISSUE(TILE_, STAGE_) do { \\\n";
-    o << "    cx::mbar_expect_tx(&bar_full[(STAGE_)], stage_tx); \\\n";
-    for (int c = 0; c < NSC; ++c)
-      o << "    if ((m_cols >> " << c << ") & 1ULL) cx::bulk_g2s(stage_buf + ((STAGE_) * NSC + " << c << ") * TR, d_" << fact_cols[c]
-        << " + (TILE_) * TR, " << TR * 4 << "u, &bar_full[(STAGE_)], l2_policy); \\\n";
-    o << "  } while (0)\n";
+    o << "  bool vec_ok = true;\n";
+    for (const auto& c : fact_cols) o << "  vec_ok = vec_ok && ((((unsigned long long)d_" << c << ") & " << VW * 4 - 1 << "ULL) == 0ULL);\n";
     o << "  __syncthreads();\n";
-    o << "  const unsigned long long m_res = s_nj[" << dims.size() << "], m_push = s_nj[" << dims.size() + 1
-      << "], m_all = s_nj[" << dims.size() + 2 << "];\n";
-    o << "  (void)m_res; (void)m_push;\n";
-    o << "  const unsigned long long m_cols = s_nj[" << dims.size() + 3 << "];\n";
-    o << "  const unsigned stage_tx = (unsigned)__popcll(m_cols) * (unsigned)(TR * 4);\n";
-    o << "  (void)stage_tx;\n";
-    // Enough (query, slice) units to occupy the aggregation warps, but no
-    // slice under 8 blocks: a small batch leaves warps idle rather than pay a
-    // flush per sliver.
-    o << "  const int slices = nq > 0 ? max(1, min((NCW + nq - 1) / nq, " << std::max(1, NB / 8) << ")) : 1;\n";
-    o << "  const int units = nq * slices;\n";
-    const std::string LIM = std::to_string(wait_limit) + "u";
-    // Per-tile views of one stage.
-    auto tile_ptrs = [&](const std::string& ind) {
-      o << ind << "const long long tile_offset = t * TR;\n";
-      o << ind << "const int n_tile = (int)(n_rows - tile_offset < TR ? n_rows - tile_offset : TR);\n";
-      o << ind << "const int nblk = (n_tile + 31) >> 5;\n";
-      o << ind << "int* tile = stage_buf + s * NSC * TR;\n";
-      for (int c = 0; c < NSC; ++c) o << ind << "const int* S_" << fact_cols[c] << " = tile + " << c << " * TR;\n";
-      for (const Dim& d : dims)
-        for (const auto& at : d.attrs)
-          o << ind << "int* S_" << at << " = s_attr + (s * " << nattr << " + " << attr_slot[at] << ") * TR;\n";
-      o << ind << "unsigned* s_qb_t = s_qb + s * nq * " << NBS << ";\n";
-      o << ind << "unsigned* s_gm_t = s_gm + s * " << gm_words * NBS << "; (void)s_gm_t;\n";
-    };
-    // Staging warp: refills a stage once the aggregation warps released it.
-    o << "  if (warp == 0) {\n";
-    o << "    if (lane == 0) {\n";
-    o << "      long long k = 0;\n";
-    o << "      for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++k) {\n";
-    o << "        const int s = (int)(k % NSTAGE);\n";
-    o << "        if (k >= NSTAGE && !cx::mbar_wait_bounded(&bar_empty[s], (unsigned)(((k / NSTAGE) - 1) & 1), " << LIM << ")) {\n";
-    o << "          cx::raise(a.err, cx::ERR_WAIT_TIMEOUT);\n";
-    o << "          *s_abort = 1;\n";
-    o << "          break;\n";
-    o << "        }\n";
-    o << "        if (*s_abort) break;\n";
-    o << "        cx::fence_proxy_async_smem();\n";
-    o << "        if (staged_ok && t < full_tiles) CX_ISSUE(t, s); else cx::mbar_arrive(&bar_full[s]);\n";
-    o << "        *s_nissued = (int)(k + 1);\n";
+    o << "  const unsigned long long m_cols = s_nj[" << ND + 3 << "];\n";
+    const unsigned long long every = NSC >= 64 ? ~0ULL : (1ULL << NSC) - 1ULL;
+    o << "  const long long n = a.rows[0];\n";
+    o << "  const long long ntiles = (n + TROWS - 1) / TROWS;\n";
+    o << "  const long long nw = (long long)gridDim.x * " << NW << ";\n";
+    // Masks of one word where the pass has at most 32 queries, of two else.
+    for (int wide = 0; wide < 2; ++wide) {
+    const std::string M = wide ? "unsigned long long" : "unsigned";
+    o << (wide ? "  } else {\n" : "  if (nq <= 32) {\n");
+    o << "  const " << M << " m_all = (" << M << ")s_nj[" << ND + 2 << "];\n";
+    for (int d = 0; d < ND; ++d) o << "  const " << M << " nj" << d << "_ = (" << M << ")s_nj[" << d << "];\n";
+    o << "  for (long long t = (long long)blockIdx.x * " << NW << " + warp; t < ntiles; t += nw) {\n";
+    // Lanes that left a tile's update loops apart would otherwise walk the
+    // following tiles apart: single warps then ran three times as long.
+    o << "    __syncwarp();\n";
+    o << "    const long long base = t * TROWS;\n";
+    o << "    const int nt = (int)(n - base < TROWS ? n - base : TROWS);\n";
+    for (const auto& c : fact_cols) o << "    int c_" << c << "[IPT];\n";
+    o << "    if (nt == TROWS && vec_ok && m_cols == " << every << "ULL) {\n";
+    for (const auto& c : fact_cols) o << "      WarpLoadTileV<IPT>(d_" << c << " + base, lane, c_" << c << ");\n";
+    o << "    } else {\n";
+    o << "      #pragma unroll\n";
+    o << "      for (int i = 0; i < IPT; ++i) {\n";
+    o << "        const int r = lane * VW + i;\n";
+    for (size_t k = 0; k < NSC; ++k)
+      o << "        c_" << fact_cols[k] << "[i] = (r < nt && ((m_cols >> " << k << ") & 1ULL)) ? d_" << fact_cols[k] << "[base + r] : 0;\n";
     o << "      }\n";
     o << "    }\n";
-    // Mask warps.
-    o << "  } else if (warp <= NPW) {\n";
-    o << "    const int pw = warp - 1;\n";
-    o << "    long long k = 0;\n";
-    o << "    for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++k) {\n";
-    o << "      const int s = (int)(k % NSTAGE);\n";
-    o << "      const bool ok_ = cx::mbar_wait_bounded(&bar_full[s], (unsigned)((k / NSTAGE) & 1), " << LIM << ");\n";
-    o << "      if (__any_sync(0xffffffffu, !ok_)) { if (lane == 0) { cx::raise(a.err, cx::ERR_WAIT_TIMEOUT); *s_abort = 1; } break; }\n";
-    o << "      if (__any_sync(0xffffffffu, *s_abort != 0)) break;\n";
-    tile_ptrs("      ");
-    o << "      const bool staged = staged_ok && t < full_tiles;\n";
-    // Phase A: query masks of the tile's rows, RB rows per thread with every
-    // dimension gather of those rows in flight together.
-    const int RB = dims.size() <= 2 ? std::min(IPT, 2) : 1;  // 64 registers hold 8 gathered entries
-    o << "    for (int b0_ = pw; b0_ < nblk; b0_ += " << NPW * RB << ") {\n";
-    // Ragged last tile (or unaligned columns): each mask warp loads the rows of its own blocks.
-    o << "      if (!staged) {\n";
-    o << "        for (int j = 0; j < " << RB << "; ++j) {\n";
-    o << "          const int r = ((b0_ + j * NPW) << 5) + lane;\n";
-    o << "          if (r >= n_tile) continue;\n";
-    for (int c = 0; c < NSC; ++c) o << "          tile[" << c << " * TR + r] = d_" << fact_cols[c] << "[tile_offset + r];\n";
-    o << "        }\n";
-    o << "        __syncwarp();\n";
-    o << "      }\n";
-    o << "      unsigned long long mk_[" << RB << "];\n";
-    o << "      bool ow_[" << RB << "];\n";
-    o << "      #pragma unroll\n";
-    o << "      for (int j = 0; j < " << RB << "; ++j) {\n";
-    o << "        const int i = ((b0_ + j * NPW) << 5) + lane;\n";
-    o << "        mk_[j] = 0ULL;\n";
-    o << "        ow_[j] = false;\n";
-    o << "        if (i < n_tile) {\n";
-    o << "          unsigned long long m = m_all;\n";
+    o << "    " << M << " m_[IPT];\n";
+    o << "    bool oow_[IPT];\n";
+    o << "    #pragma unroll\n";
+    o << "    for (int i = 0; i < IPT; ++i) {\n";
+    o << "      " << M << " m = lane * VW + i < nt ? m_all : (" << M << ")0;\n";
+    o << "      oow_[i] = false;\n";
     for (int k = 0; k < NFC; ++k) {
       const int ck = (int)(std::find(fact_cols.begin(), fact_cols.end(), fcols[k]) - fact_cols.begin());
-      o << "          if ((m_cols >> " << ck << ") & 1ULL) { const unsigned d_ = (unsigned)S_" << fcols[k] << "[i] - fb" << k << ";\n";
-      o << "            if (d_ < fw" << k << ") m &= s_fm[" << k * FW << " + d_]; else ow_[j] = true; }\n";
+      o << "      if ((m_cols >> " << ck << ") & 1ULL) { const unsigned d_ = (unsigned)c_" << fcols[k] << "[i] - fb" << k << ";\n";
+      o << "        if (d_ < fw" << k << ") m &= (" << M << ")s_fm[" << k * FW << " + d_]; else oow_[i] = true; }\n";
     }
-    o << "          mk_[j] = m;\n";
-    o << "        }\n";
-    o << "      }\n";
-    for (size_t di = 0; di < dims.size(); ++di) o << "      int4 g" << di << "_[" << RB << "];\n";
-    for (size_t di = 0; di < dims.size(); ++di) o << "      int k" << di << "_[" << RB << "];\n";
-    o << "      #pragma unroll\n";
-    o << "      for (int j = 0; j < " << RB << "; ++j) {\n";
-    o << "        const int i = ((b0_ + j * NPW) << 5) + lane;\n";
-    o << "        const bool live_ = i < n_tile && mk_[j] != 0ULL;\n";
-    for (size_t di = 0; di < dims.size(); ++di) {
-      const Dim& d = dims[di];
-      o << "        {\n";
-      o << "          g" << di << "_[j] = make_int4(0, 0, 0, 0);\n";
-      o << "          const int fk_ = live_ ? S_" << d.fk << "[i] : 0;\n";
-      o << "          k" << di << "_[j] = fk_;\n";
-      o << "          const int h_ = cx_detail::pht_slot<int>(fk_, " << d.len << ", " << d.keymin << ");\n";
-      o << "          if (live_ && h_ >= 0) g" << di << "_[j] = __ldg(&dkm_" << lower(d.name) << "[h_]);\n";
-      o << "        }\n";
-    }
-    o << "      }\n";
-    o << "      #pragma unroll\n";
-    o << "      for (int j = 0; j < " << RB << "; ++j) {\n";
-    o << "        const int i = ((b0_ + j * NPW) << 5) + lane;\n";
-    o << "        if (b0_ + j * NPW >= nblk) break;  // warp-uniform: a block is one warp's 32 rows\n";
-    o << "        unsigned long long m = mk_[j];\n";
-    o << "        const bool oow = ow_[j]; (void)oow;\n";
-    o << "        if (m != 0ULL) {\n";
+    o << "      m_[i] = m;\n";
+    o << "    }\n";
+    // Dimensions: those whose entries stay in L1 first, then the others.
+    for (const Dim& d : dims)
+      for (const auto& at : d.attrs) o << "    int S_" << at << "[IPT];\n";
     const char* comp[] = {"x", "y", "z"};
-    for (size_t di = 0; di < dims.size(); ++di) {
-      const Dim& d = dims[di];
-      const std::string dn = lower(d.name);
-      o << "          {\n";
-      o << "            const int4 g_ = g" << di << "_[j];\n";
-      o << "            const bool hit_ = g_.x != 0 && g_.x == k" << di << "_[j];\n";
-      o << "            m &= hit_ ? (((unsigned long long)(unsigned)g_.z << 32) | (unsigned)g_.y) : s_nj[" << di << "];\n";
-      if (!d.attrs.empty()) o << "            S_" << d.attrs[0] << "[i] = g_.w;\n";
-      if (d.attrs.size() > 1) {
-        o << "            int4 a_ = make_int4(0, 0, 0, 0);\n";
-        o << "            if (hit_) a_ = __ldg(&dat_" << dn << "[cx_detail::pht_slot<int>(k" << di << "_[j], " << d.len << ", " << d.keymin << ")]);\n";
-        for (size_t k = 1; k < d.attrs.size(); ++k) o << "            S_" << d.attrs[k] << "[i] = a_." << comp[k - 1] << ";\n";
+    for (int phase = 0; phase < 2; ++phase) {
+      std::vector<int> now;
+      for (int di = 0; di < ND; ++di)
+        if ((dims[di].len * 16 <= (1LL << 20)) == (phase == 0)) now.push_back(di);
+      if (now.empty()) continue;
+      o << "    {\n";
+      for (int di : now) o << "      int4 g" << di << "_[IPT];\n";
+      o << "      #pragma unroll\n";
+      o << "      for (int i = 0; i < IPT; ++i) {\n";
+      for (int di : now) {
+        const Dim& d = dims[di];
+        o << "        { const int h_ = (m_[i] & ~nj" << di << "_) ? cx_detail::pht_slot<int>(c_" << d.fk << "[i], " << d.len << ", " << d.keymin << ") : -1;\n";
+        o << "          g" << di << "_[i] = h_ >= 0 ? " << (phase == 0 ? "__ldg" : "__ldcg") << "(&dkm_" << lower(d.name) << "[h_]) : make_int4(0, 0, 0, 0); }\n";
       }
-      o << "          }\n";
+      o << "      }\n";
+      o << "      #pragma unroll\n";
+      o << "      for (int i = 0; i < IPT; ++i) {\n";
+      for (int di : now) {
+        const Dim& d = dims[di];
+        o << "        { const int4 g_ = g" << di << "_[i];\n";
+        o << "          const bool hit_ = g_.x != 0 && g_.x == c_" << d.fk << "[i];\n";
+        o << "          m_[i] &= hit_ ? " << (wide ? "(((unsigned long long)(unsigned)g_.z << 32) | (unsigned)g_.y)" : "(unsigned)g_.y") << " : nj" << di << "_;\n";
+        if (!d.attrs.empty()) o << "          S_" << d.attrs[0] << "[i] = g_.w;\n";
+        if (d.attrs.size() > 1) {
+          o << "          int4 a_ = make_int4(0, 0, 0, 0);\n";
+          o << "          if (hit_ && (m_[i] & ~nj" << di << "_)) a_ = __ldg(&dat_" << lower(d.name) << "[cx_detail::pht_slot<int>(c_" << d.fk << "[i], "
+            << d.len << ", " << d.keymin << ")]);\n";
+          for (size_t k = 1; k < d.attrs.size(); ++k) o << "          S_" << d.attrs[k] << "[i] = a_." << comp[k - 1] << ";\n";
+        }
+        o << "        }\n";
+      }
+      o << "      }\n";
+      o << "    }\n";
     }
+    auto map_cols = [&](Emitter& e) {
+      for (const auto& c : fact_cols) e.col_expr[c] = "c_" + c + "[i]";
+      for (const Dim& d : dims)
+        for (const auto& at : d.attrs) e.col_expr[at] = "S_" + at + "[i]";
+    };
+    o << "    #pragma unroll\n";
+    o << "    for (int i = 0; i < IPT; ++i) {\n";
+    o << "      " << M << " m = m_[i];\n";
     // Residual filters (and filter-table conjuncts of values outside the window).
     bool any_slow = false;
-    for (size_t s = 0; s < shapes.size(); ++s) any_slow = any_slow || !preds[s].resid.empty() || !preds[s].pushed.empty();
+    for (int s = 0; s < NSH; ++s) any_slow = any_slow || !preds[s].resid.empty() || !preds[s].pushed.empty();
     if (any_slow) {
-      o << "        unsigned long long r_ = m & (m_res | (oow ? m_push : 0ULL));\n";
-      o << "        while (r_) {\n";
-      o << "          const int q = __ffsll((long long)r_) - 1;\n";
-      o << "          r_ &= r_ - 1ULL;\n";
-      o << "          const int* P = s_params + s_sq[q].param_off; (void)P;\n";
-      o << "          bool pass = true;\n";
-      o << "          switch (s_sq[q].shape) {\n";
-      for (size_t s = 0; s < shapes.size(); ++s) {
+      o << "      const bool oow = oow_[i];\n";
+      o << "      " << M << " r_ = m & (" << M << ")(s_nj[" << ND << "] | (oow ? s_nj[" << ND + 1 << "] : 0ULL));\n";
+      o << "      while (r_) {\n";
+      o << "        const int q = " << (wide ? "__ffsll((long long)r_)" : "__ffs((int)r_)") << " - 1;\n";
+      o << "        r_ &= r_ - 1;\n";
+      o << "        const int* P = s_params + s_sq[q].param_off; (void)P;\n";
+      o << "        bool pass = true;\n";
+      o << "        switch (s_sq[q].shape) {\n";
+      for (int s = 0; s < NSH; ++s) {
         if (preds[s].resid.empty() && preds[s].pushed.empty()) continue;
         Emitter e(*shapes[s], tu);
         e.lit_index = &lit_maps[s];
-        for (const auto& c : fact_cols) e.col_expr[c] = "S_" + c + "[i]";
-        for (const auto& kv : attr_slot) e.col_expr[kv.first] = "S_" + kv.first + "[i]";
+        map_cols(e);
         std::vector<const Expr*> all_pushed;
         for (const auto& kv : preds[s].pushed) all_pushed.insert(all_pushed.end(), kv.second.begin(), kv.second.end());
-        o << "            case " << s << ": pass = (" << conj_and(e, preds[s].resid) << ") && (!oow || (" << conj_and(e, all_pushed) << ")); break;\n";
+        o << "          case " << s << ": pass = (" << conj_and(e, preds[s].resid) << ") && (!oow || (" << conj_and(e, all_pushed) << ")); break;\n";
       }
-      o << "            default: break;\n";
-      o << "          }\n";
-      o << "          if (!pass) m &= ~(1ULL << q);\n";
+      o << "          default: break;\n";
       o << "        }\n";
+      o << "        if (!pass) m &= ~((" << M << ")1 << q);\n";
+      o << "      }\n";
     }
-    o << "        }\n";
-    o << "        const int blk_ = i >> 5;\n";
-    for (size_t si = 0; si < shapes.size(); ++si) {
-      if (gm_base[si] < 0) continue;
-      const Plan& p = *shapes[si];
-      Emitter e(p, tu);
-      for (const auto& c : fact_cols) e.col_expr[c] = "S_" + c + "[i]";
-      for (const auto& kv : attr_slot) e.col_expr[kv.first] = "S_" + kv.first + "[i]";
-      const unsigned long long G = e.total_groups();
-      std::string horner, dom;
-      o << "        {  // group rows of shape " << si << "\n";
-      o << "          int h_ = " << G << ";\n";
-      o << "          bool bad_ = false;\n";
-      o << "          if (m != 0ULL) {\n";
-      for (size_t k = 0; k < p.groups.size(); ++k) {
-        o << "            const int gt" << k << " = " << e.group_term(k) << ";\n";
-        horner = horner.empty() ? "gt0" : "(" + horner + " * " + std::to_string(e.eff_card(k)) + " + gt" + std::to_string(k) + ")";
-        dom += (dom.empty() ? "" : " && ") + std::string("(unsigned)gt") + std::to_string(k) + " < " + std::to_string(e.eff_card(k)) + "u";
-      }
-      o << "            bad_ = !(" << dom << ");\n";
-      o << "            const int hash = bad_ ? (" << horner << ") % " << G << " : (" << horner << ");\n";
-      o << "            h_ = (unsigned)hash < " << G << "u ? hash : " << G << ";\n";
-      o << "          }\n";
-      // One match over the lanes gives every group's row word at once: the
-      // block's words are cleared, then the lowest lane of each group writes
-      // its group's word (the same lane writes the out-of-domain word).
-      const std::string gm_at = "s_gm_t[(" + std::to_string(gm_base[si]) + " + ";
-      o << "          if (lane <= " << G << ") " << gm_at << "lane) * " << NBS << " + blk_] = 0u;\n";
-      o << "          __syncwarp();\n";
-      o << "          const unsigned peers_ = __match_any_sync(0xffffffffu, h_);\n";
-      o << "          if (h_ < " << G << " && lane == __ffs(peers_) - 1) " << gm_at << "h_) * " << NBS << " + blk_] = peers_;\n";
-      o << "          const unsigned bb_ = __ballot_sync(0xffffffffu, bad_);\n";
-      o << "          if (lane == " << G << ") " << gm_at << G << ") * " << NBS << " + blk_] = bb_;\n";
-      o << "        }\n";
-    }
-    // Transpose the warp's 32 row masks into one word per query.
-    o << "        const unsigned wl_ = cx::warp_transpose32((unsigned)m, lane);\n";
-    o << "        if (lane < nq) s_qb_t[lane * " << NBS << " + blk_] = wl_;\n";
-    o << "        if (nq > 32) {\n";
-    o << "          const unsigned wh_ = cx::warp_transpose32((unsigned)(m >> 32), lane);\n";
-    o << "          if (lane + 32 < nq) s_qb_t[(lane + 32) * " << NBS << " + blk_] = wh_;\n";
-    o << "        }\n";
-    o << "      }\n";
-    o << "    }\n";
-    o << "    __syncwarp();\n";
-    o << "    if (lane == 0) cx::mbar_arrive(&bar_ready[s]);\n";
-    o << "    }\n";
-    // Aggregation warps: query units aggregate the rows whose bit is set.
-    o << "  } else {\n";
-    o << "    const int cw = warp - 1 - NPW;\n";
-    o << "    long long k = 0;\n";
-    o << "    for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++k) {\n";
-    o << "      const int s = (int)(k % NSTAGE);\n";
-    o << "      const bool ok_ = cx::mbar_wait_bounded(&bar_ready[s], (unsigned)((k / NSTAGE) & 1), " << LIM << ");\n";
-    o << "      if (__any_sync(0xffffffffu, !ok_)) { if (lane == 0) { cx::raise(a.err, cx::ERR_WAIT_TIMEOUT); *s_abort = 1; } break; }\n";
-    o << "      if (__any_sync(0xffffffffu, *s_abort != 0)) break;\n";
-    tile_ptrs("      ");
-    o << "    for (int u = cw; u < units; u += NCW) {\n";
-    o << "      const int q_ = u / slices, sl_ = u - q_ * slices;\n";
-    o << "      const int perb_ = (nblk + slices - 1) / slices;\n";
-    o << "      const int blo_ = sl_ * perb_, bhi_ = blo_ + perb_ < nblk ? blo_ + perb_ : nblk;\n";
-    // Fewer blocks than lanes: lanes share a block, each taking a bit range of its word.
-    o << "      const int lpb_ = perb_ >= 32 ? 1 : perb_ >= 16 ? 2 : perb_ >= 8 ? 4 : perb_ >= 4 ? 8 : perb_ >= 2 ? 16 : 32;\n";
-    o << "      const int bw_ = 32 / lpb_, sub_ = lane % lpb_;\n";
-    o << "      const unsigned bm_ = (bw_ == 32 ? 0xffffffffu : ((1u << bw_) - 1u)) << (sub_ * bw_);\n";
-    o << "      const CxSQ& Q = s_sq[q_];\n";
-    o << "      const int* P = s_params + Q.param_off; (void)P;\n";
-    o << "      const unsigned* qw_ = s_qb_t + q_ * " << NBS << ";\n";
-    o << "      switch (Q.shape) {\n";
-    for (size_t s = 0; s < shapes.size(); ++s) {
+    // A shape's queries are neighbouring bits: half a mask word of them at a time.
+    for (int s = 0; s < NSH; ++s) {
       const Plan& p = *shapes[s];
       Emitter e(p, tu);
       e.lit_index = &lit_maps[s];
-      const std::string ind = "          ";
-      o << "      case " << s << ": {\n";
-      const int NA = (int)p.aggs.size();
-      const int TS = p.storage_ts();
-      std::vector<std::string> need;
-      for (const auto& g : p.groups) cols_of(g.expr.get(), need);
-      for (const auto& ag : p.aggs) cols_of(ag.arg.get(), need);
-      // Parameters of group and aggregate expressions in registers.
-      {
-        std::vector<const Expr*> ls;
-        for (const auto& g : p.groups) lits_of(g.expr.get(), ls);
-        for (const auto& ag : p.aggs) lits_of(ag.arg.get(), ls);
-        std::set<int> ks;
-        for (const Expr* l : ls) ks.insert(lit_maps[s].at(l));
-        for (int k : ks) o << ind << "const int P" << k << " = P[" << k << "];\n";
-      }
-      e.param_regs = true;
-      for (const auto& c : need) e.col_expr[c] = "S_" + c + "[i]";
-      // Each lane walks the set bits of its 32-row blocks.
-      std::string loop_open = ind + "for (int b_ = blo_ + lane / lpb_; b_ < bhi_; b_ += 32 / lpb_) {\n";
-      loop_open += ind + "  unsigned w_ = qw_[b_] & bm_;\n";
-      loop_open += ind + "  while (w_) {\n";
-      loop_open += ind + "  const int i = (b_ << 5) + __ffs(w_) - 1;\n";
-      loop_open += ind + "  w_ &= w_ - 1u;\n";
-      const std::string loop_close = ind + "  }\n" + ind + "}\n";
-      if (p.groups.empty()) {
-        for (int k = 0; k < NA; ++k) o << ind << "unsigned long long s" << k << "_ = 0ULL, c" << k << "_ = 0ULL;\n";
-        o << loop_open;
-        for (int k = 0; k < NA; ++k) {
-          const Agg& ag = p.aggs[k];
-          const std::string x = ag.fn == AggFn::Count ? "1ULL" : e.math_push(ag.arg.get(), true);
-          o << ind << "  s" << k << "_ += " << x << "; c" << k << "_ += 1ULL;\n";
-        }
-        o << loop_close;
-        for (int k = 0; k < NA; ++k) {
-          o << ind << "if (__any_sync(0xffffffffu, c" << k << "_ != 0ULL)) {\n";
-          o << ind << "  for (int o_ = 16; o_ > 0; o_ >>= 1) { s" << k << "_ += __shfl_xor_sync(0xffffffffu, s" << k << "_, o_); c" << k << "_ += __shfl_xor_sync(0xffffffffu, c" << k << "_, o_); }\n";
-          o << ind << "  if (lane == 0) { atomicAdd(&s_qacc[(long long)q_ * " << NACC << " + " << 2 * k << "], s" << k << "_); atomicAdd(&s_qacc[(long long)q_ * " << NACC << " + " << 2 * k + 1 << "], c" << k << "_); }\n";
-          o << ind << "}\n";
-        }
-      } else {
-        const unsigned long long G = e.total_groups();
-        const unsigned long long TWq = (G + 31) / 32;
-        std::string horner, dom;
-        std::ostringstream terms;
-        for (size_t k = 0; k < p.groups.size(); ++k) {
-          terms << ind << "  const int gt" << k << " = " << e.group_term(k) << ";\n";
-          horner = horner.empty() ? "gt0" : "(" + horner + " * " + std::to_string(e.eff_card(k)) + " + gt" + std::to_string(k) + ")";
-          dom += (dom.empty() ? "" : " && ") + std::string("(unsigned)gt") + std::to_string(k) + " < " + std::to_string(e.eff_card(k)) + "u";
-        }
-        o << ind << "unsigned long long* d_result = Q.result; (void)d_result;\n";
-        o << ind << "uint64_t* d_result_validity = (uint64_t*)Q.validity; (void)d_result_validity;\n";
-        o << ind << "unsigned int* g_touch = Q.touched; (void)g_touch;\n";
-        o << ind << "unsigned long long* qtab = Q.smem_acc >= 0 ? s_tab + Q.smem_acc : nullptr; (void)qtab;\n";
-        o << ind << "unsigned int* qbits = s_bits + (Q.smem_acc >= 0 ? Q.smem_bits : 0); (void)qbits;\n";
-        // Flush of a unit's register partials: one reduce-scatter of all G x NA
-        // values; the lanes that end up holding a total apply it.
-        auto tiny_flush = [&]() {
-          int P2 = 1;
-          while (P2 < (int)(G * NA)) P2 <<= 1;
-          o << ind << "ttouch = __reduce_or_sync(0xffffffffu, ttouch);\n";
-          for (int k = 0; k < NA; ++k)
-            if (!p.sparse && p.aggs[k].fn == AggFn::Sum) o << ind << "tseen" << k << " = __reduce_or_sync(0xffffffffu, tseen" << k << ");\n";
-          o << ind << "if (ttouch) {\n";
-          o << ind << "  unsigned long long rv_[" << P2 << "];\n";
-          o << ind << "  #pragma unroll\n" << ind << "  for (int r = 0; r < " << P2 << "; ++r) rv_[r] = r < " << G * NA << " ? tacc[r < " << G * NA << " ? r : 0] : 0ULL;\n";
-          o << ind << "  const int ri_ = cx::warp_reduce_scatter_u64<" << P2 << ">(rv_, lane);\n";
-          o << ind << "  const int g = ri_ / " << NA << ", k_ = ri_ - g * " << NA << "; (void)k_;\n";
-          o << ind << "  if ((lane & " << (32 / P2 - 1) << ") == 0 && ri_ < " << G * NA << " && ((ttouch >> g) & 1u)) {\n";
-          o << ind << "    const unsigned long long s_ = rv_[0];\n";
-          int sk = 0;
-          for (int k = 0; k < NA; ++k) {
-            const int slot = (int)p.groups.size() + k;
-            const std::string ix = "(unsigned long long)g * " + std::to_string(TS) + "ULL + " + std::to_string(slot);
-            o << ind << "    if (k_ == " << k << ") {\n";
-            o << ind << "      if (qtab) { if (s_) atomicAdd(&qtab[ri_], s_); }\n";
-            o << ind << "      else if (s_) atomicAdd(&d_result[" << ix << "], s_);\n";
-            if (!p.sparse) {
-              if (p.aggs[k].fn == AggFn::Count) o << ind << "      if (!qtab) db::atomic_set_valid_bit(d_result_validity, " << ix << ");\n";
-              else {
-                o << ind << "      if ((tseen" << k << " >> g) & 1u) { if (qtab) atomicOr(&qbits[" << TWq * (1 + sk) << "ULL + (g >> 5)], 1u << (g & 31)); else db::atomic_set_valid_bit(d_result_validity, " << ix << "); }\n";
-                ++sk;
-              }
-            }
-            o << ind << "    }\n";
-          }
-          o << ind << "  }\n";
-          o << ind << "  if (lane == 0) { if (qtab) atomicOr(&qbits[0], ttouch); else atomicOr(&g_touch[0], ttouch); }\n";
-          o << ind << "}\n";
-        };
-        if (gm_base[s] >= 0) {
-          // Group row bitmaps: per block and group, the query's rows of that
-          // group; COUNT is a popcount, SUM walks the rows.
-          o << ind << "unsigned long long tacc[" << G * NA << "];\n";
-          o << ind << "#pragma unroll\n" << ind << "for (int r = 0; r < " << G * NA << "; ++r) tacc[r] = 0ULL;\n";
-          o << ind << "unsigned ttouch = 0u;\n";
-          o << ind << "const unsigned* gm_ = s_gm_t + " << gm_base[s] << " * " << NBS << ";\n";
-          o << ind << "for (int b_ = blo_ + lane / lpb_; b_ < bhi_; b_ += 32 / lpb_) {\n";
-          o << ind << "  const unsigned w_ = qw_[b_] & bm_;\n";
-          o << ind << "  if (!w_) continue;\n";
-          o << ind << "  if (w_ & gm_[" << G << " * " << NBS << " + b_]) cx::raise(a.err, cx::ERR_GROUP_DOMAIN);\n";
-          o << ind << "  #pragma unroll\n";
-          o << ind << "  for (int g = 0; g < " << G << "; ++g) {\n";
-          o << ind << "    unsigned wg_ = w_ & gm_[g * " << NBS << " + b_];\n";
-          o << ind << "    if (!wg_) continue;\n";
-          o << ind << "    ttouch |= 1u << g;\n";
-          bool any_sum = false;
-          for (int k = 0; k < NA; ++k) {
-            if (p.aggs[k].fn == AggFn::Count) o << ind << "    tacc[g * " << NA << " + " << k << "] += (unsigned long long)__popc(wg_);\n";
-            else any_sum = true;
-          }
-          if (any_sum) {
-            o << ind << "    while (wg_) {\n";
-            o << ind << "      const int i = (b_ << 5) + __ffs(wg_) - 1;\n";
-            o << ind << "      wg_ &= wg_ - 1u;\n";
-            for (int k = 0; k < NA; ++k)
-              if (p.aggs[k].fn == AggFn::Sum)
-                o << ind << "      tacc[g * " << NA << " + " << k << "] += (unsigned long long)(" << e.math_push(p.aggs[k].arg.get(), true) << ");\n";
-            o << ind << "    }\n";
-          }
-          o << ind << "  }\n";
-          o << ind << "}\n";
-          // No nullable columns in a shared shape: a SUM is valid wherever its group was touched.
-          for (int k = 0; k < NA; ++k)
-            if (!p.sparse && p.aggs[k].fn == AggFn::Sum) o << ind << "unsigned tseen" << k << " = ttouch;\n";
-          tiny_flush();
-        } else {
-        const bool tiny = G <= 32 && G * (unsigned long long)NA <= 16;
-        if (tiny && tu.group_merge == 2) {
-          // Queries with a shared-memory table add straight into it; the
-          // touched / seen bits collect in registers until the unit ends.
-          o << ind << "if (qtab) {\n";
-          o << ind << "unsigned ttouch = 0u;\n";
-          for (int k = 0; k < NA; ++k)
-            if (!p.sparse && p.aggs[k].fn == AggFn::Sum) o << ind << "unsigned tseen" << k << " = 0u;\n";
-          o << loop_open;
-          o << terms.str();
-          o << ind << "  int hash = " << horner << ";\n";
-          o << ind << "  if (!(" << dom << ")) { cx::raise(a.err, cx::ERR_GROUP_DOMAIN); hash = hash % " << G << "; }\n";
-          o << ind << "  if ((unsigned)hash >= " << G << "u) continue;\n";
-          o << ind << "  ttouch |= 1u << hash;\n";
-          for (int k = 0; k < NA; ++k) {
-            const Agg& ag = p.aggs[k];
-            const std::string x = ag.fn == AggFn::Count ? "1ULL" : "(unsigned long long)(" + e.math_push(ag.arg.get(), true) + ")";
-            o << ind << "  { const unsigned long long x_ = " << x << "; if (x_) atomicAdd(&qtab[hash * " << NA << " + " << k << "], x_); }\n";
-            if (!p.sparse && ag.fn == AggFn::Sum) o << ind << "  tseen" << k << " |= 1u << hash;\n";
-          }
-          o << loop_close;
-          o << ind << "ttouch = __reduce_or_sync(0xffffffffu, ttouch);\n";
-          int sk = 0;
-          for (int k = 0; k < NA; ++k)
-            if (!p.sparse && p.aggs[k].fn == AggFn::Sum) {
-              o << ind << "tseen" << k << " = __reduce_or_sync(0xffffffffu, tseen" << k << ");\n";
-              o << ind << "if (lane == 0 && tseen" << k << ") atomicOr(&qbits[" << TWq * (1 + sk) << "], tseen" << k << ");\n";
-              ++sk;
-            }
-          o << ind << "if (lane == 0 && ttouch) atomicOr(&qbits[0], ttouch);\n";
-          o << ind << "} else {\n";
-        }
-        if (tiny) {
-          o << ind << "unsigned long long tacc[" << G * NA << "];\n";
-          o << ind << "#pragma unroll\n" << ind << "for (int r = 0; r < " << G * NA << "; ++r) tacc[r] = 0ULL;\n";
-          o << ind << "unsigned ttouch = 0u;\n";
-          for (int k = 0; k < NA; ++k)
-            if (!p.sparse && p.aggs[k].fn == AggFn::Sum) o << ind << "unsigned tseen" << k << " = 0u;\n";
-        }
-        if (tiny) {
-          o << loop_open;
-          o << terms.str();
-          o << ind << "  int hash = " << horner << ";\n";
-          o << ind << "  if (!(" << dom << ")) { cx::raise(a.err, cx::ERR_GROUP_DOMAIN); hash = hash % " << G << "; }\n";
-          o << ind << "  if ((unsigned)hash >= " << G << "u) continue;\n";
-          o << ind << "  ttouch |= 1u << hash;\n";
-          for (int k = 0; k < NA; ++k) {
-            const Agg& ag = p.aggs[k];
-            const std::string x = ag.fn == AggFn::Count ? "1ULL" : "(unsigned long long)(" + e.math_push(ag.arg.get(), true) + ")";
-            o << ind << "  { const unsigned long long x_ = " << x << ";\n";
-            o << ind << "    #pragma unroll\n" << ind << "    for (int g = 0; g < " << G << "; ++g) if (hash == g) tacc[g * " << NA << " + " << k << "] += x_;\n";
-            if (!p.sparse && ag.fn == AggFn::Sum) o << ind << "    tseen" << k << " |= 1u << hash;\n";
-            o << ind << "  }\n";
-          }
-          o << loop_close;
-          tiny_flush();
-          if (tu.group_merge == 2) o << ind << "}\n";
-        } else if (tu.group_merge == 2 || tu.group_merge == 3) {
-          // Direct per-row updates: shared-memory table when the query has one, else global atomics.
-          o << loop_open;
-          o << terms.str();
-          o << ind << "  int hash = " << horner << ";\n";
-          o << ind << "  if (!(" << dom << ")) { cx::raise(a.err, cx::ERR_GROUP_DOMAIN); hash = hash % " << G << "; }\n";
-          o << ind << "  if ((unsigned)hash >= " << G << "u) continue;\n";
-          o << ind << "  if (qtab) {\n";
-          o << ind << "    atomicOr(&qbits[hash >> 5], 1u << (hash & 31));\n";
-          int sk = 0;
-          for (int k = 0; k < NA; ++k) {
-            const Agg& ag = p.aggs[k];
-            const std::string x = ag.fn == AggFn::Count ? "1ULL" : "(unsigned long long)(" + e.math_push(ag.arg.get(), true) + ")";
-            o << ind << "    { const unsigned long long x_ = " << x << "; if (x_) atomicAdd(&qtab[(long long)hash * " << NA << " + " << k << "], x_);";
-            if (!p.sparse && ag.fn == AggFn::Sum) { o << " atomicOr(&qbits[" << TWq * (1 + sk) << "ULL + (hash >> 5)], 1u << (hash & 31));"; ++sk; }
-            o << " }\n";
-          }
-          o << ind << "  } else {\n";
-          o << ind << "    atomicOr(&g_touch[hash >> 5], 1u << (hash & 31));\n";
-          for (int k = 0; k < NA; ++k) {
-            const Agg& ag = p.aggs[k];
-            const int slot = (int)p.groups.size() + k;
-            const std::string ix = "(unsigned long long)hash * " + std::to_string(TS) + "ULL + " + std::to_string(slot);
-            const std::string x = ag.fn == AggFn::Count ? "1ULL" : "(unsigned long long)(" + e.math_push(ag.arg.get(), true) + ")";
-            o << ind << "    { const unsigned long long x_ = " << x << "; if (x_) atomicAdd(&d_result[" << ix << "], x_);";
-            if (!p.sparse && ag.fn == AggFn::Sum) o << " db::atomic_set_valid_bit(d_result_validity, " << ix << ");";
-            o << " }\n";
-            if (!p.sparse && ag.fn == AggFn::Count) o << ind << "    db::atomic_set_valid_bit(d_result_validity, " << ix << ");\n";
-          }
-          o << ind << "  }\n";
-          o << loop_close;
-        } else {
-          // Larger domains: one row per lane per round in a warp-uniform loop;
-          // lanes that hit the same group merge their values (one
-          // `__match_any_sync`) so the table sees one atomic per distinct
-          // group, not one per row -- a query's few live groups would
-          // otherwise serialise the warp's atomics.
-          o << ind << "int b_ = blo_ + lane / lpb_;\n";
-          o << ind << "unsigned w_ = b_ < bhi_ ? (qw_[b_] & bm_) : 0u;\n";
-          o << ind << "for (;;) {\n";
-          o << ind << "  while (w_ == 0u && b_ < bhi_) { b_ += 32 / lpb_; w_ = b_ < bhi_ ? (qw_[b_] & bm_) : 0u; }\n";
-          o << ind << "  if (!__any_sync(0xffffffffu, w_ != 0u)) break;\n";
-          o << ind << "  int hash = -1;\n";
-          for (int k = 0; k < NA; ++k) o << ind << "  unsigned long long x" << k << "_ = 0ULL;\n";
-          o << ind << "  if (w_ != 0u) {\n";
-          o << ind << "  const int i = (b_ << 5) + __ffs(w_) - 1;\n";
-          o << ind << "  w_ &= w_ - 1u;\n";
-          o << terms.str();
-          o << ind << "  hash = " << horner << ";\n";
-          o << ind << "  if (!(" << dom << ")) { cx::raise(a.err, cx::ERR_GROUP_DOMAIN); hash = hash % " << G << "; }\n";
-          for (int k = 0; k < NA; ++k) {
-            const Agg& ag = p.aggs[k];
-            const std::string x = ag.fn == AggFn::Count ? "1ULL" : "(unsigned long long)(" + e.math_push(ag.arg.get(), true) + ")";
-            o << ind << "  x" << k << "_ = " << x << ";\n";
-          }
-          o << ind << "  }\n";
-          o << ind << "  const bool ok_ = (unsigned)hash < " << G << "u;\n";
-          o << ind << "  const unsigned okm_ = __ballot_sync(0xffffffffu, ok_);\n";
-          o << ind << "  if (ok_) {\n";
-          o << ind << "    const unsigned peers_ = __match_any_sync(okm_, hash);\n";
-          o << ind << "    if (__popc(peers_) > 1) {\n";
-          for (int k = 0; k < NA; ++k) {
-            o << ind << "      { unsigned long long r_ = 0ULL;\n";
-            o << ind << "        for (unsigned m_ = peers_; m_; m_ &= m_ - 1u) r_ += __shfl_sync(peers_, x" << k << "_, __ffs(m_) - 1);\n";
-            o << ind << "        x" << k << "_ = r_; }\n";
-          }
-          o << ind << "    }\n";
-          o << ind << "    if (lane == __ffs(peers_) - 1) {\n";
-          o << ind << "      if (qtab) {\n";
-          o << ind << "        atomicOr(&qbits[hash >> 5], 1u << (hash & 31));\n";
-          int sk = 0;
-          for (int k = 0; k < NA; ++k) {
-            const Agg& ag = p.aggs[k];
-            o << ind << "        if (x" << k << "_) atomicAdd(&qtab[(long long)hash * " << NA << " + " << k << "], x" << k << "_);\n";
-            if (!p.sparse && ag.fn == AggFn::Sum) { o << ind << "        atomicOr(&qbits[" << TWq * (1 + sk) << "ULL + (hash >> 5)], 1u << (hash & 31));\n"; ++sk; }
-          }
-          o << ind << "      } else {\n";
-          o << ind << "        atomicOr(&g_touch[hash >> 5], 1u << (hash & 31));\n";
-          for (int k = 0; k < NA; ++k) {
-            const Agg& ag = p.aggs[k];
-            const int slot = (int)p.groups.size() + k;
-            const std::string ix = "(unsigned long long)hash * " + std::to_string(TS) + "ULL + " + std::to_string(slot);
-            o << ind << "        if (x" << k << "_) atomicAdd(&d_result[" << ix << "], x" << k << "_);\n";
-            if (!p.sparse && (ag.fn == AggFn::Sum || ag.fn == AggFn::Count))
-              o << ind << "        db::atomic_set_valid_bit(d_result_validity, " << ix << ");\n";
-          }
-          o << ind << "      }\n";
-          o << ind << "    }\n";
-          o << ind << "  }\n";
-          o << ind << "}\n";
-        }
-        }
-      }
-      o << "        break; }\n";
-    }
-    o << "        default: break;\n";
-    o << "      }\n";
-    o << "    }\n";
-    o << "    __syncwarp();\n";
-    o << "    if (lane == 0) cx::mbar_arrive(&bar_empty[s]);\n";
-    o << "    }\n";
-    o << "  }\n";
-    o << "  __syncthreads();\n";
-    // After a timeout: wait (bounded) for the copies still in flight, then leave.
-    o << "  if (*s_abort) {\n";
-    o << "    if (threadIdx.x == 0 && staged_ok) {\n";
-    o << "      const int ni = *s_nissued;\n";
-    o << "      for (int kk = ni - NSTAGE < 0 ? 0 : ni - NSTAGE; kk < ni; ++kk)\n";
-    o << "        if ((long long)blockIdx.x + (long long)kk * gridDim.x < full_tiles)\n";
-    o << "          (void)cx::mbar_wait_bounded(&bar_full[kk % NSTAGE], (unsigned)((kk / NSTAGE) & 1), cx::drain_limit_us(" << LIM << "));\n";
-    o << "    }\n";
-    o << "    return;\n";
-    o << "  }\n";
-    o << "  for (int q = threadIdx.x; q < nq; q += " << CTA << ") {\n";
-    o << "    const CxSQ& Q = s_sq[q];\n";
-    o << "    switch (Q.shape) {\n";
-    for (size_t s = 0; s < shapes.size(); ++s) {
-      const Plan& p = *shapes[s];
-      if (!p.groups.empty()) continue;
-      o << "      case " << s << ": {\n";
-      for (size_t k = 0; k < p.aggs.size(); ++k) {
-        o << "        { const unsigned long long s_ = s_qacc[(long long)q * " << NACC << " + " << 2 * k << "], c_ = s_qacc[(long long)q * " << NACC << " + " << 2 * k + 1 << "];\n";
-        o << "          if (s_) atomicAdd(&Q.result[" << k << "], s_);\n";
-        if (p.aggs[k].fn == AggFn::Count) o << "          db::atomic_set_valid_bit((uint64_t*)Q.validity, " << k << ");\n";
-        else o << "          if (c_) db::atomic_set_valid_bit((uint64_t*)Q.validity, " << k << ");\n";
-        o << "        }\n";
-      }
-      o << "        break; }\n";
-    }
-    o << "      default: break;\n";
-    o << "    }\n";
-    o << "  }\n";
-    // Grouped queries with shared-memory tables: one flush per CTA.
-    o << "  for (int q = 0; q < nq; ++q) {\n";
-    o << "    const CxSQ& Q = s_sq[q];\n";
-    o << "    if (Q.smem_acc < 0) continue;\n";
-    o << "    unsigned long long* d_result = Q.result; (void)d_result;\n";
-    o << "    uint64_t* d_result_validity = (uint64_t*)Q.validity; (void)d_result_validity;\n";
-    o << "    const unsigned long long* qtab = s_tab + Q.smem_acc;\n";
-    o << "    const unsigned int* qbits = s_bits + Q.smem_bits;\n";
-    o << "    switch (Q.shape) {\n";
-    for (size_t s2 = 0; s2 < shapes.size(); ++s2) {
-      const Plan& p = *shapes[s2];
-      if (p.groups.empty()) continue;
-      Emitter e(p, tu);
+      map_cols(e);
+      const QTab qt = qtab_of(p);
       const unsigned long long G = e.total_groups();
-      const int NA = (int)p.aggs.size();
-      if (G * (unsigned long long)NA * 8 > 4096ULL) continue;
-      const unsigned long long TWq = (G + 31) / 32;
-      const int TS = p.storage_ts();
-      o << "      case " << s2 << ":\n";
-      o << "        for (long long g = threadIdx.x; g < " << G << "LL; g += " << CTA << ") {\n";
-      o << "          if (!((qbits[g >> 5] >> (g & 31)) & 1u)) continue;\n";
-      e.emit_key_store(o, "g", "          ");
-      int sk = 0;
-      for (int k = 0; k < NA; ++k) {
-        const int slot = (int)p.groups.size() + k;
-        const std::string ix = "(unsigned long long)g * " + std::to_string(TS) + "ULL + " + std::to_string(slot);
-        o << "          { const unsigned long long v_ = qtab[g * " << NA << " + " << k << "];\n";
-        o << "            if (v_) atomicAdd(&d_result[" << ix << "], v_);\n";
-        if (!p.sparse) {
-          if (p.aggs[k].fn == AggFn::Count) o << "            db::atomic_set_valid_bit(d_result_validity, " << ix << ");\n";
-          else {
-            o << "            if ((qbits[" << TWq * (1 + sk) << "ULL + (g >> 5)] >> (g & 31)) & 1u) db::atomic_set_valid_bit(d_result_validity, " << ix << ");\n";
-            ++sk;
+      const int TS = p.storage_ts(), NA = (int)p.aggs.size(), NG = (int)p.groups.size();
+      // Group and values once per row where they hold no literal, else per query.
+      std::vector<const Expr*> ls;
+      for (const auto& g : p.groups) lits_of(g.expr.get(), ls);
+      for (const auto& ag : p.aggs) lits_of(ag.arg.get(), ls);
+      const bool per_query = !ls.empty();
+      std::ostringstream val;
+      std::string horner, dom;
+      for (int k = 0; k < NG; ++k) {
+        val << "          const int gt" << k << " = " << e.group_term(k) << ";\n";
+        horner = horner.empty() ? "gt0" : "(" + horner + " * " + std::to_string(e.eff_card(k)) + " + gt" + std::to_string(k) + ")";
+        dom += (dom.empty() ? "" : " && ") + std::string("(unsigned)gt") + std::to_string(k) + " < " + std::to_string(e.eff_card(k)) + "u";
+      }
+      if (NG) {
+        val << "          int hash = " << horner << ";\n";
+        val << "          if (" << (per_query ? "" : "b_ != 0u && ") << "!(" << dom << ")) { cx::raise(a.err, cx::ERR_GROUP_DOMAIN); hash = hash % " << G << "; }\n";
+      } else {
+        val << "          const int hash = 0;\n";
+      }
+      for (int k = 0; k < NA; ++k)
+        if (p.aggs[k].fn == AggFn::Sum)
+          val << "          const unsigned long long x" << k << "_ = (unsigned long long)(" << e.math_push(p.aggs[k].arg.get(), true) << ");\n";
+      o << "      for (int h_ = 0; h_ < a.sq_num[" << s << "]; h_ += 32) {\n";
+      o << "        const int q0_ = a.sq_first[" << s << "] + h_, nb_ = a.sq_num[" << s << "] - h_;\n";
+      o << "        unsigned b_ = (unsigned)(m >> q0_) & (nb_ >= 32 ? ~0u : (1u << nb_) - 1u);\n";
+      o << "        if (!__any_sync(0xffffffffu, b_ != 0u)) continue;\n";
+      if (!per_query) {
+        o << val.str();
+        if (NG) o << "          if ((unsigned)hash >= " << G << "u) b_ = 0u;\n";
+      }
+      // One query per lane and round, the warp together: loops that lanes leave
+      // one by one left some warps' lanes apart for good (a warp then ran three
+      // times as long as the others).
+      o << "        while (__any_sync(0xffffffffu, b_ != 0u)) {\n";
+      o << "          if (b_ == 0u) continue;\n";
+      o << "          const int q = q0_ + __ffs((int)b_) - 1;\n";
+      o << "          b_ &= b_ - 1u;\n";
+      if (per_query) {
+        o << "          const int* P = s_params + s_sq[q].param_off; (void)P;\n";
+        o << val.str();
+        o << "          if ((unsigned)hash >= " << G << "u) continue;\n";
+      }
+      if (qt.u64) {
+        o << "          const int2 qt_ = s_qt[q];\n";
+        o << "          if (qt_.x >= 0) {\n";
+        o << "            unsigned* w_ = s_tab + qt_.x + (unsigned)hash * " << qt.words * qt.rep << "u"
+          << (qt.rep > 1 ? " + (lane & " + std::to_string(qt.rep - 1) + ")" : std::string()) << ";\n";
+        int w = 0;
+        bool first = true;
+        for (int k = 0; k < NA; ++k) {
+          if (p.aggs[k].fn == AggFn::Count) {
+            o << "            atomicAdd(&w_[" << w++ * qt.rep << "], 1u);\n";
+            continue;
           }
+          const std::string x = "x" + std::to_string(k) + "_";
+          o << "            { const unsigned xl_ = (unsigned)" << x << ", old_ = atomicAdd(&w_[" << w * qt.rep << "], xl_);\n";
+          o << "              const unsigned xh_ = (unsigned)(" << x << " >> 32) + (old_ + xl_ < xl_ ? 1u : 0u);\n";
+          o << "              if (xh_) atomicAdd(&w_[" << (w + 1) * qt.rep << "], xh_);\n";
+          // The first row of a copy finds its low word 0.
+          if (first && !qt.counts) o << "              if (old_ == 0u) cx::set_bit_once(&s_bits[qt_.y + (hash >> 5)], 1u << (hash & 31));\n";
+          o << "            }\n";
+          first = false;
+          w += 2;
         }
+        o << "            continue;\n";
         o << "          }\n";
       }
+      o << "          unsigned long long* r_ = s_sq[q].result + (unsigned long long)hash * " << TS << "ULL + " << NG << ";\n";
+      for (int k = 0; k < NA; ++k) {
+        if (p.aggs[k].fn == AggFn::Count) o << "          atomicAdd(&r_[" << k << "], 1ULL);\n";
+        else o << "          atomicAdd(&r_[" << k << "], x" << k << "_);\n";
+      }
+      if (NG) o << "          cx::set_bit_once(&s_sq[q].touched[hash >> 5], 1u << (hash & 31));\n";
+      else o << "          cx::set_valid_bits((uint64_t*)s_sq[q].validity, 0ULL, " << (NA >= 64 ? ~0ULL : (1ULL << NA) - 1ULL) << "ULL);\n";
+      o << "        }\n";
+      o << "      }\n";
+    }
+    o << "    }\n";
+    o << "  }\n";
+    }
+    o << "  }\n";
+    // The tables into the results, once per CTA: a warp per group where every
+    // lane has its copy (queries start at different warps), else a thread.  The
+    // key kernel afterwards writes keys and validity of the touched groups.
+    o << "  __syncthreads();\n";
+    o << "  for (int q = 0; q < nq; ++q) {\n";
+    o << "    const CxSQ& Q = s_sq[q];\n";
+    o << "    const unsigned* qb_ = s_bits + s_qt[q].y; (void)qb_;\n";
+    o << "    if (s_qt[q].x < 0) continue;\n";
+    o << "    switch (Q.shape) {\n";
+    for (int s = 0; s < NSH; ++s) {
+      const Plan& p = *shapes[s];
+      const QTab qt = qtab_of(p);
+      if (!qt.u64) continue;
+      Emitter e(p, tu);
+      const unsigned long long G = e.total_groups();
+      const int TS = p.storage_ts(), NA = (int)p.aggs.size(), NG = (int)p.groups.size();
+      const bool by_warp = qt.rep == 32;
+      o << "      case " << s << ":\n";
+      if (by_warp) o << "        for (int g = (warp + q) % " << NW << "; g < " << G << "; g += " << NW << ") {\n";
+      else o << "        for (int g = threadIdx.x; g < " << G << "; g += " << CTA << ") {\n";
+      if (!qt.counts) o << "          if (!((qb_[g >> 5] >> (g & 31)) & 1u)) continue;\n";
+      o << "          const unsigned* w_ = s_tab + s_qt[q].x + (unsigned)g * " << qt.words * qt.rep << "u;\n";
+      int w = 0;
+      std::string any;
+      for (int k = 0; k < NA; ++k) {
+        const bool sum = p.aggs[k].fn == AggFn::Sum;
+        const std::string v = "v" + std::to_string(k) + "_";
+        auto at = [&](const std::string& r) {
+          const std::string lo = "w_[" + std::to_string(w * qt.rep) + " + " + r + "]";
+          return sum ? "cx::lohi(" + lo + ", w_[" + std::to_string((w + 1) * qt.rep) + " + " + r + "])" : "(unsigned long long)" + lo;
+        };
+        if (by_warp) o << "          const unsigned long long " << v << " = cx::warp_sum_u64(" << at("lane") << ");\n";
+        else o << "          unsigned long long " << v << " = 0ULL;\n          for (int r = 0; r < " << qt.rep << "; ++r) " << v << " += " << at("r") << ";\n";
+        if (!sum && any.empty()) any = v;
+        w += sum ? 2 : 1;
+      }
+      if (qt.counts) o << "          if (!" << any << ") continue;\n";
+      if (by_warp) o << "          if (lane != 0) continue;\n";
+      for (int k = 0; k < NA; ++k)
+        o << "          if (v" << k << "_) atomicAdd(&Q.result[(unsigned long long)g * " << TS << "ULL + " << NG + k << "], v" << k << "_);\n";
+      if (NG) o << "          cx::set_bit_once(&Q.touched[g >> 5], 1u << (g & 31));\n";
+      else o << "          cx::set_valid_bits((uint64_t*)Q.validity, 0ULL, " << (NA >= 64 ? ~0ULL : (1ULL << NA) - 1ULL) << "ULL);\n";
       o << "        }\n        break;\n";
     }
     o << "      default: break;\n";
     o << "    }\n";
     o << "  }\n";
-    o << "}\n";
-    o << "#undef CX_ISSUE\n\n";
+    o << "}\n\n";
   }
 
   void emit_keys() {
@@ -4096,13 +3729,22 @@ struct SharedGen {
     src << "  switch (Q.shape) {\n";
     for (size_t s = 0; s < shapes.size(); ++s) {
       const Plan& p = *shapes[s];
-      if (p.groups.empty()) continue;
       Emitter e(p, tu);
+      if (p.groups.empty()) {
+        // One row in any case: a COUNT is valid, a SUM where a row was added (set with it).
+        src << "    case " << s << ":\n";
+        for (size_t k = 0; k < p.aggs.size(); ++k)
+          if (p.aggs[k].fn == AggFn::Count)
+            src << "      if (threadIdx.x == 0) db::atomic_set_valid_bit(d_result_validity, " << k << ");\n";
+        src << "      break;\n";
+        continue;
+      }
       src << "    case " << s << ":\n";
       src << "      for (long long g = (long long)(blockIdx.x % a.zero_parts) * 256 + threadIdx.x; g < " << e.total_groups()
           << "LL; g += (long long)a.zero_parts * 256) {\n";
       src << "        if (!((Q.touched[g >> 5] >> (g & 31)) & 1u)) continue;\n";
-      e.emit_key_store(src, "g", "        ");
+      // No nullable columns in a shared shape: every aggregate of a touched group is valid.
+      e.emit_group_row(src, "g", "        ", std::vector<std::string>(p.aggs.size(), "1"));
       src << "      }\n      break;\n";
     }
     src << "    default: break;\n  }\n}\n\n";

@@ -137,7 +137,7 @@ struct LaunchPlan {
   bool rows_sized = false;                             // some hash table is sized by a table's rows
   std::map<int, uint64_t> dat_words;                   // shared scans: extra payload attributes per dimension
   std::vector<std::pair<int, std::string>> fcols;      // shared scans: fact filter table columns
-  struct SShape { uint64_t groups; int ts, grouped, sparse, nlits, smem_ok, naggs; uint64_t tw; int nseen; };
+  struct SShape { uint64_t groups; int ts, grouped, sparse, nlits, smem_ok, naggs; uint64_t tw; int nseen; uint64_t tab = 0, bits = 0; };
   std::vector<SShape> sshapes;
   // Shared scans with an aggregate-cube path: its attributes (dimension index
   // and 16-bit field of the entry, or dim -1 for a fact column) and, per shape,
@@ -219,6 +219,12 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
     } else if (k == "sshape") {
       int i; LaunchPlan::SShape sh;
       ls >> i >> sh.groups >> sh.ts >> sh.grouped >> sh.sparse >> sh.nlits >> sh.smem_ok >> sh.naggs >> sh.tw >> sh.nseen;
+      // A query's shared-memory table (u64 words, 0: none) and presence bits (u32 words).
+      if (!ls.fail() && !(ls >> sh.tab >> sh.bits)) {
+        ls.clear();
+        sh.tab = sh.smem_ok ? sh.groups * (uint64_t)sh.naggs : 0;
+        sh.bits = sh.smem_ok ? sh.tw * (uint64_t)(1 + sh.nseen) : 0;
+      }
       if (i != (int)lp.sshapes.size()) { err = "shape lines out of order"; return false; }
       lp.sshapes.push_back(sh);
     } else if (k == "cube") {
@@ -1724,9 +1730,9 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
       hsq[j].smem_acc = -1;
       hsq[j].smem_bits = 0;
       hsq[j].keep = keep ? (keep[order[q0 + j]] ? 1 : 0) : 0;
-      if (cube || !sh.smem_ok) continue;
-      const uint64_t tw = tab_words + sh.groups * (uint64_t)sh.naggs;
-      const uint64_t bw = bit_words + sh.tw * (uint64_t)(1 + sh.nseen);
+      if (cube || !sh.tab) continue;
+      const uint64_t tw = tab_words + sh.tab;
+      const uint64_t bw = bit_words + sh.bits;
       if (sk.smem + qb_bytes + tw * 8 + bw * 4 + 64 > smem_cap) continue;
       hsq[j].smem_acc = (int)tab_words;
       hsq[j].smem_bits = (int)bit_words;
