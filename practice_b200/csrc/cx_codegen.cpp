@@ -878,6 +878,28 @@ struct Emitter {
         W32 += (ag.fn == AggFn::Count ? 0 : 2) + (ag.fn == AggFn::Sum ? 0 : cnt_words);
       }
     }
+    // "Any valid input" of a SUM / MIN / MAX in those tables: a value that cannot
+    // be NULL has one wherever its group was touched; one with the validity of a
+    // COUNT or AVG wherever that count is not zero; the others keep a bitmap, one
+    // for all with the same validity.  seen_as: -1 touched, >= 0 that aggregate's
+    // count, -2 - k the bitmap of aggregate k.
+    std::vector<int> seen_as(NA, -1);
+    {
+      const std::set<std::string> keep = valid_regs;
+      for (const auto& c : p.nullable) valid_regs.insert(c);
+      std::vector<std::string> v(NA);
+      for (int k = 0; k < NA; ++k) v[k] = p.aggs[k].arg->op == Op::Star ? "1" : valid_of(p.aggs[k].arg.get());
+      valid_regs = keep;
+      for (int k = 0; k < NA; ++k) {
+        if (seen_idx[k] < 0 || lit_true(v[k])) continue;
+        seen_as[k] = -2 - k;
+        for (int q = NA - 1; q >= 0; --q) {
+          if (v[q] != v[k]) continue;
+          if (seen_as[k] < 0 && q < k && seen_idx[q] >= 0) seen_as[k] = -2 - q;
+          if (p.aggs[q].fn == AggFn::Count || p.aggs[q].fn == AggFn::Avg) seen_as[k] = q;
+        }
+      }
+    }
     int LREP = 1;
     if (grouped && !reg_groups && !lane_groups) {
       const unsigned long long one = G * NACC * 8 + TW * 4 * (1 + NSEEN_T);
@@ -1396,37 +1418,35 @@ struct Emitter {
     // and MIN / MAX before they are lowered / raised; a stale read costs an
     // atomic that changes nothing.  A COUNT(*) stands in for the touched bit.
     const int star_slot = count_star_slot();
-    auto w32_update = [&](const std::string& ii) {
-      auto set_bit = [&](const std::string& words) {
-        o << ii << "cx::set_bit_once(&" << words << ", 1u << (hash & 31));\n";
+    // (`on`: a bool expression the updates are predicated by, empty = none.)
+    auto w32_update = [&](const std::string& ii, const std::string& on = "") {
+      auto guard = [&](const std::string& v) {
+        const std::string c = on.empty() ? v : lit_true(v) ? on : on + " && (" + v + ")";
+        return lit_true(c) ? std::string() : "if (" + c + ") ";
       };
       o << ii << "unsigned* w_ = cx_w32 + (unsigned)hash * " << W32 * LREP << "u"
         << (LREP > 1 ? " + (lane & " + std::to_string(LREP - 1) + ")" : std::string()) << ";\n";
-      if (star_slot < 0) set_bit("s_touch[hash >> 5]");
+      if (star_slot < 0) o << ii << guard("1") << "cx::set_bit_once(&s_touch[hash >> 5], 1u << (hash & 31));\n";
       for (int k = 0; k < NA; ++k) {
         const Agg& ag = p.aggs[k];
-        const std::string v = ag.arg->op == Op::Star ? "1" : valid_of(ag.arg.get());
+        const std::string g = guard(ag.arg->op == Op::Star ? "1" : valid_of(ag.arg.get()));
         auto word = [&](int w) { return "&w_[" + std::to_string(w * LREP) + "]"; };
         const int w0 = w32_word[k];
         auto count = [&](int w) {
-          if (cnt_words == 1) o << ii << "  atomicAdd(" << word(w) << ", 1u);\n";
-          else o << ii << "  cx::add_lohi(" << word(w) << ", " << word(w + 1) << ", 1ULL);\n";
+          if (cnt_words == 1) o << ii << g << "atomicAdd(" << word(w) << ", 1u);\n";
+          else o << ii << g << "cx::add_lohi(" << word(w) << ", " << word(w + 1) << ", 1ULL);\n";
         };
-        o << ii << "if (" << v << ") {\n";
         switch (ag.fn) {
           case AggFn::Count: count(w0); break;
-          case AggFn::Min: o << ii << "  cx::min_word(" << word(w0) << ", (unsigned)" << math_push(ag.arg.get(), false) << ");\n"; break;
-          case AggFn::Max: o << ii << "  cx::max_word(" << word(w0) << ", (unsigned)" << math_push(ag.arg.get(), false) << ");\n"; break;
+          case AggFn::Min: o << ii << g << "cx::min_word(" << word(w0) << ", (unsigned)" << math_push(ag.arg.get(), false) << ");\n"; break;
+          case AggFn::Max: o << ii << g << "cx::max_word(" << word(w0) << ", (unsigned)" << math_push(ag.arg.get(), false) << ");\n"; break;
           default:
-            o << ii << "  cx::add_lohi(" << word(w0) << ", " << word(w0 + 1) << ", (unsigned long long)("
+            o << ii << g << "cx::add_lohi(" << word(w0) << ", " << word(w0 + 1) << ", (unsigned long long)("
               << math_push(ag.arg.get(), true) << "));\n";
             if (ag.fn == AggFn::Avg) count(w0 + 2);
         }
-        if (seen_idx[k] >= 0 && NSEEN_T > 0) {
-          o << ii << "  ";
-          o << "cx::set_bit_once(&s_seen[" << (unsigned long long)seen_idx[k] * TW << "u + (hash >> 5)], 1u << (hash & 31));\n";
-        }
-        o << ii << "}\n";
+        if (seen_idx[k] >= 0 && NSEEN_T > 0 && seen_as[k] == -2 - k)
+          o << ii << g << "cx::set_bit_once(&s_seen[" << (unsigned long long)seen_idx[k] * TW << "u + (hash >> 5)], 1u << (hash & 31));\n";
       }
     };
     auto item_consume = [&](const std::string& ii) {
@@ -1779,6 +1799,44 @@ struct Emitter {
         o << ii << "}\n";
       }
     };
+    // An OR-join followed by nothing but filters and a shared-memory group table:
+    // every branch of every item is one predicate and predicated updates, no
+    // nested branches (60M rows into 12 groups, COUNT / MIN / MAX / AVG over a
+    // nullable column: 0.427 -> 0.420 ms, and 0.3635 with the seen bits of NULL-able
+    // values read off their counts).
+    bool flat_or = expanding && !p.steps[xs].join.multi && w32;
+    for (size_t k = xs + 1; k < p.steps.size(); ++k) flat_or = flat_or && p.steps[k].kind == Step::Filter;
+    auto flat_branches = [&](const std::string& ii) {
+      const Join& j = p.steps[xs].join;
+      o << ii << "#pragma unroll\n" << ii << "for (int i = 0; i < ITEMS_PER_THREAD; ++i) {\n";
+      for (size_t f = 0; f < j.fks.size(); ++f) {
+        const std::string F = std::to_string(f), i2 = ii + "    ";
+        o << ii << "  {\n";
+        if (!j.payload.empty()) o << i2 << j.payload << "[i] = cx_or_pay" << F << "_[i];\n";
+        if (!j.payload.empty() && payload_valid.count(j.payload))
+          o << i2 << j.payload << "_valid[i] = (int)((cx_or_val" << F << "_ >> i) & 1u);\n";
+        o << i2 << "bool cx_on = ((cx_or_hit >> (i * " << j.fks.size() << " + " << F << ")) & 1u) != 0u;\n";
+        {
+          EagerScope eager;
+          for (size_t k = xs + 1; k < p.steps.size(); ++k) {
+            const std::string c = and_terms({valid_of(p.steps[k].filter.get()), value_of(p.steps[k].filter.get())});
+            if (!lit_true(c)) o << i2 << "cx_on = cx_on & (bool)(" << c << ");\n";
+          }
+        }
+        std::string horner, dom;
+        for (size_t k = 0; k < p.groups.size(); ++k) {
+          o << i2 << "const int gt" << k << " = " << group_term(k) << ";\n";
+          horner = horner.empty() ? "gt0" : "(" + horner + " * " + std::to_string(eff_card(k)) + " + gt" + std::to_string(k) + ")";
+          dom += (dom.empty() ? "" : " && ") + std::string("(unsigned)gt") + std::to_string(k) + " < " + std::to_string(eff_card(k)) + "u";
+        }
+        o << i2 << "int hash = " << horner << ";\n";
+        o << i2 << "if (cx_on && !(" << dom << ")) { cx::raise(a.err, cx::ERR_GROUP_DOMAIN); hash = hash % " << G << "; }\n";
+        o << i2 << "cx_on = cx_on && (unsigned)hash < " << G << "u;\n";
+        w32_update(i2, "cx_on");
+        o << ii << "  }\n";
+      }
+      o << ii << "}\n";
+    };
     // Aggregate consume.
     auto emit_consume = [&](const std::string& ind) {
       if (uniform_expand) {
@@ -1786,6 +1844,7 @@ struct Emitter {
       } else if (expanding) {
         if (probe_first) mht_probes(ind);
         else if (!p.steps[xs].join.multi) or_probes(ind);
+        if (flat_or) return flat_branches(ind);
         o << ind << "#pragma unroll\n" << ind << "for (int i = 0; i < ITEMS_PER_THREAD; ++i) {\n";
         o << ind << "  if (flags[i] && (tid + BLOCK_THREADS * i < num_tile_items)) {\n";
         item_steps(xs, ind + "    ");
@@ -2018,8 +2077,11 @@ struct Emitter {
         std::vector<std::string> seen(NA);
         for (int k = 0; k < NA; ++k) {
           if (p.aggs[k].fn == AggFn::Count) seen[k] = "1";
-          else if (seen_idx[k] >= 0 && !p.sparse)
-            seen[k] = "(s_seen[" + std::to_string((unsigned long long)seen_idx[k] * TW) + "u + (g >> 5)] >> (g & 31)) & 1u";
+          if (seen_idx[k] < 0 || p.sparse) continue;
+          const int as = seen_as[k];
+          if (as == -1) seen[k] = "1";
+          else if (as >= 0) seen[k] = std::string(p.aggs[as].fn == AggFn::Avg ? "c" : "v") + std::to_string(as) + "_ != 0ULL";
+          else seen[k] = "(s_seen[" + std::to_string((unsigned long long)seen_idx[-2 - as] * TW) + "u + (g >> 5)] >> (g & 31)) & 1u";
         }
         emit_group_row(o, "g", "    ", seen);
       }
