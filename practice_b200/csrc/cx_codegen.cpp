@@ -1354,11 +1354,13 @@ struct Emitter {
         o << ii << "}\n";
       }
     };
-    auto lane_update = [&](const std::string& ii) {
-      o << ii << "rtouch |= 1u << hash;\n";
+    // (`on`: a bool expression the update is predicated by, empty = none.)
+    auto lane_update = [&](const std::string& ii, const std::string& on = "") {
+      o << ii << (on.empty() ? "" : "if (" + on + ") ") << "rtouch |= 1u << hash;\n";
       for (int k = 0; k < NA; ++k) {
         const Agg& ag = p.aggs[k];
-        const std::string v = ag.arg->op == Op::Star ? "1" : valid_of(ag.arg.get());
+        const std::string va = ag.arg->op == Op::Star ? "1" : valid_of(ag.arg.get());
+        const std::string v = on.empty() ? va : lit_true(va) ? on : on + " && (" + va + ")";
         const std::string x = ag.fn == AggFn::Count ? "1ULL" : "(unsigned long long)(" + math_push(ag.arg.get(), true) + ")";
         const std::string r = "s_lacc[((unsigned)hash * " + std::to_string(NACC) + "u + " + std::to_string(k) + "u) * " +
                               std::to_string(CTA) + "u + threadIdx.x]";
@@ -1804,7 +1806,7 @@ struct Emitter {
     // nested branches (60M rows into 12 groups, COUNT / MIN / MAX / AVG over a
     // nullable column: 0.427 -> 0.420 ms, and 0.3635 with the seen bits of NULL-able
     // values read off their counts).
-    bool flat_or = expanding && !p.steps[xs].join.multi && w32;
+    bool flat_or = expanding && !p.steps[xs].join.multi && (w32 || lane_groups);
     for (size_t k = xs + 1; k < p.steps.size(); ++k) flat_or = flat_or && p.steps[k].kind == Step::Filter;
     auto flat_branches = [&](const std::string& ii) {
       const Join& j = p.steps[xs].join;
@@ -1832,7 +1834,8 @@ struct Emitter {
         o << i2 << "int hash = " << horner << ";\n";
         o << i2 << "if (cx_on && !(" << dom << ")) { cx::raise(a.err, cx::ERR_GROUP_DOMAIN); hash = hash % " << G << "; }\n";
         o << i2 << "cx_on = cx_on && (unsigned)hash < " << G << "u;\n";
-        w32_update(i2, "cx_on");
+        if (w32) w32_update(i2, "cx_on");
+        else lane_update(i2, "cx_on");
         o << ii << "  }\n";
       }
       o << ii << "}\n";
