@@ -821,7 +821,7 @@ struct Emitter {
         if (s.kind != Step::JoinStep) continue;
         const bool table = ptable.count(s.join.dim) > 0;
         if (!table && !bitmaps.count(s.join.dim)) continue;
-        const unsigned long long words = (unsigned long long)(table ? (s.join.len + 3) / 4 : (s.join.len + 31) / 32);
+        const unsigned long long words = (unsigned long long)(table ? (s.join.len + 3) / 4 : s.join.len / 32 + 1);
         off = (off + 15) & ~15ULL;
         sbms.push_back({s.join.dim, s.join.fks[0], ht_slot.at(s.join.dim), s.join.len, s.join.keymin, words, off,
                         !s.join.payload.empty(), table, s.join.prange_min});
@@ -1240,7 +1240,7 @@ struct Emitter {
           << ", flags, (const unsigned char*)s_bm_" << lower(b.dim) << ", " << ht_name(b.dim) << ", " << b.len << ", "
           << b.keymin << ", num_tile_items);\n";
       else
-        o << ind << "BlockProbeExactBitmap<int, BLOCK_THREADS, ITEMS_PER_THREAD>(tid, " << b.fk << ", flags, s_bm_"
+        o << ind << "BlockProbeExactBitmapPad<int, BLOCK_THREADS, ITEMS_PER_THREAD>(tid, " << b.fk << ", flags, s_bm_"
           << lower(b.dim) << ", " << ht_name(b.dim) << ", " << (b.pair ? 1 : 0) << ", " << b.len << ", " << b.keymin
           << ", num_tile_items);\n";
       exact_dims.insert(b.dim);
@@ -2251,7 +2251,7 @@ struct Emitter {
       if (!s.join.payload.empty() && payload_valid.count(s.join.payload))
         meta << "htv " << h << " " << (s.join.len + 31) / 32 << "\n";
       if (ptable.count(s.join.dim)) meta << "bm " << h << " " << (s.join.len + 3) / 4 << "\n";
-      else if (bitmaps.count(s.join.dim)) meta << "bm " << h << " " << (s.join.len + 31) / 32 << "\n";
+      else if (bitmaps.count(s.join.dim)) meta << "bm " << h << " " << s.join.len / 32 + 1 << "\n";  // (bit len is 0)
       ++h;
     }
     if (h > CX_MAX_HTS_) throw PlanError("too many joins");
