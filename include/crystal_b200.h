@@ -58,8 +58,8 @@ typedef struct cx_tuning {
                             default 48 KiB) */
   int group_merge;       /* 0 auto, 1 merge equal groups within a warp first (for a plan with one
                             OR / multi-value join: a warp-uniform expansion loop), 2 per-lane
-                            atomics, 3 shared scans: per-row atomics above 32 groups only */
-  int producer_warps;    /* shared scans: warps that build query masks (0 = 3/8 of the block) */
+                            atomics; shared scans update per row whatever it is */
+  int producer_warps;    /* accepted and not used: every warp of a shared scan builds masks */
   int parametric;        /* plain kernels: 1 = integer literals become launch parameters
                             (one module per plan shape, literals passed to cx_execute_params) */
   int prefetch;          /* unstaged plain scans (stages = 0): 0 = each column loaded where the
@@ -234,8 +234,10 @@ int cx_plan_literals(const char* plan, size_t plan_len, int64_t* out, int cap, i
  * shape; its literals are ignored).  Same output contract as cx_codegen; fails
  * with CX_E_INVALID for shapes that cannot share a scan (nullable columns,
  * aggregates other than COUNT/SUM, conflicting joins, OR-joins, multi-value
- * hash joins).  A NULL tuning means 1024 threads, 1 row per thread, 3 staging
- * stages, 1 CTA per SM. */
+ * hash joins).  A NULL tuning means 1024 threads, 1 row per thread, 3 stages,
+ * 1 CTA per SM.  Items per thread and stages only bound the launch shape (tiles
+ * of block x items rows, `stages` of them, must fit 200 KB of shared memory);
+ * the mask scan takes two rows a lane from registers, the cube scan `cube`. */
 int cx_shared_codegen(const char* const* plans, const size_t* plan_lens, int nshapes, const cx_tuning* tuning,
                       char* out, size_t out_cap, size_t* out_len);
 /* Enqueues one batch (<= 256 queries, <= 4096 parameters) of a compiled shared
@@ -323,7 +325,9 @@ typedef struct cx_sort_key {
 /* Writes the result rows column by column: column c at dev_columns + c *
  * row_cap, its validity bits at dev_col_validity + c * ((row_cap + 63) / 64).
  * row_cap must cover the group count.  `limit` = UINT64_MAX for none.  Returns
- * the number of rows in *rows (synchronises `stream`). */
+ * the number of rows in *rows (synchronises `stream`).  Its scratch comes
+ * stream-ordered from a pool of the library's own, one per device, which keeps
+ * at most 32 MiB between calls. */
 int cx_finalize(const uint64_t* dev_result, const uint64_t* dev_validity, const cx_result_layout* layout,
                 const cx_sort_key* keys, int nkeys, uint64_t limit, uint64_t* dev_columns,
                 uint64_t* dev_col_validity, uint64_t row_cap, uint64_t* rows, void* stream);

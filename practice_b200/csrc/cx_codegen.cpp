@@ -3415,6 +3415,30 @@ struct SharedGen {
     return t;
   }
 
+  // Shared memory that tiles of block x items rows, `stages` of them, would
+  // take with their payloads and row bitmaps: launch shapes above 200 KB are
+  // refused, as callers that try shapes in turn expect.  (The scan below keeps
+  // its rows in registers whatever the shape.)
+  unsigned long long staged_bytes() const {
+    const unsigned long long TR = (unsigned long long)tu.block_threads * tu.items_per_thread, NB = TR / 32;
+    unsigned long long nattr = 0, words = 0, S = std::max(2, tu.stages);
+    for (const Dim& d : dims) nattr += d.attrs.size();
+    for (const Plan* p : shapes) {
+      if (p->groups.empty() || tu.group_merge == 2) continue;
+      Emitter e(*p, tu);
+      const unsigned long long G = e.total_groups();
+      std::vector<const Expr*> gl;
+      for (const auto& g : p->groups) lits_of(g.expr.get(), gl);
+      if (G <= 31 && G * p->aggs.size() <= 16 && gl.empty()) words += G + 1;
+    }
+    while (S > 2 && S * ((fact_cols.size() + nattr) * TR * 4 + (MAXQ + words) * NB * 4) > 160 * 1024) --S;
+    auto up = [](unsigned long long x) { return (x + 15) & ~15ULL; };
+    unsigned long long off = up(S * ((fact_cols.size() + nattr) * TR * 4 + words * (NB + 1) * 4 + 24) + 16);
+    off = up(off + (unsigned long long)MAXQ * std::max(1, max_lits) * 4) + (unsigned long long)MAXQ * std::max(1, max_scalar_aggs) * 16;
+    off += up((unsigned long long)MAXQ * sizeof(CxSQ)) + (unsigned long long)fcols.size() * FW * 8 + (dims.size() + 4) * 8;
+    return up(off) + MAXQ * S * (NB + 1) * 4;
+  }
+
   // Shared scan by per-query row masks.  Every warp walks tiles of 32 x IPT
   // rows: per row the mask of the queries that keep it (filter tables, then one
   // gather per dimension, small dimensions first so that rows no query joins
@@ -3431,6 +3455,7 @@ struct SharedGen {
     const int CTA = tu.block_threads;
     if (CTA % 32 || CTA < 64 || CTA > 1024 || tu.items_per_thread < 1 || tu.items_per_thread > 16) throw PlanError("bad block shape");
     if (CTA / 32 < 3) throw PlanError("shared scan needs at least 3 warps");
+    if (staged_bytes() > 200 * 1024) throw PlanError("shared scan shared memory exceeds 200 KB before group tables");
     const int IPT = 2, VW = 2, NW = CTA / 32;
     const int MAXP = MAXQ * std::max(1, max_lits);
     const int NFC = (int)fcols.size(), ND = (int)dims.size(), NSH = (int)shapes.size();

@@ -20,9 +20,8 @@ struct Tuning {
   int smem_group_budget = 96 * 1024;  // bytes of shared memory a group table may use
   int bitmap_budget = 48 * 1024;      // bytes of shared memory for join membership bitmaps
   int group_merge = 0;         // 0 auto, 1 warp match-merge (one expanding join: warp-uniform
-                               // expansion), 2 direct per-lane atomics, 3 shared scans: direct
-                               // per-row atomics above 32 groups only
-  int producer_warps = 0;      // shared scans: warps that build query masks (0 = 3/8 of the block)
+                               // expansion), 2 direct per-lane atomics
+  int producer_warps = 0;      // accepted and not used
   int parametric = 0;          // plain kernels: literals read from CxArgs.lits at run time
   int prefetch = 1;            // unstaged plain scans: 0 columns loaded where first used,
                                // 1 vector loads of every column at the tile start,

@@ -70,8 +70,7 @@ DEFAULT_CANDIDATES = [
 ]
 
 
-# Shared-scan launch shape before autotuning: one 32-warp CTA per SM, 1024-row
-# tiles, a three-stage ring.
+# Shared-scan launch shape before autotuning: one 32-warp CTA per SM.
 SHARED_DEFAULT = dict(block_threads=1024, items_per_thread=1, stages=3, ctas_per_sm=1)
 
 
