@@ -849,7 +849,8 @@ struct Emitter {
     }
     // Shared-memory group tables of 32-bit words: a SUM is a low and a high word
     // (the carry of the low add goes into the high one), a COUNT one word (two
-    // where a multi-value join can repeat a row without bound), MIN / MAX of an
+    // where a multi-value join can repeat a row without bound; else `rowmax` in
+    // the launch plan bounds the rows of one launch), MIN / MAX of an
     // int32 column one word (sign extension keeps the unsigned order).  32-bit
     // shared atomics are native; 64-bit ones are compare-and-swap loops, and
     // merging equal groups across the warp first (__match_any_sync, then a
@@ -863,7 +864,12 @@ struct Emitter {
     // 0.345 -> 0.306 ms unqueued, three joins into 175 groups 0.203 -> 0.195 ms.
     // group_merge = 1 and MIN / MAX over expressions keep the 64-bit tables.
     bool any_multi = false;
-    for (const auto& s : p.steps) any_multi = any_multi || (s.kind == Step::JoinStep && s.join.multi);
+    unsigned long long or_rows = 1;  // most times the OR-joins let one fact row count
+    for (const auto& s : p.steps) {
+      if (s.kind != Step::JoinStep) continue;
+      any_multi = any_multi || s.join.multi;
+      or_rows *= s.join.fks.size();
+    }
     std::vector<int> w32_word(NA, 0);  // first word of each aggregate
     int W32 = 0;
     bool w32 = grouped && !reg_groups && !lane_groups && tu.group_merge != 1;
@@ -981,6 +987,11 @@ struct Emitter {
     const unsigned wait_limit = (unsigned)std::min(60000000, std::max(1, tu.wait_limit_us));
 
     const std::string kname = "Scan_" + fact;
+    // Counts of one 32-bit word per CTA: the host launches no more rows at a time
+    // than such a word can count (0: none, any number of rows).
+    bool counts32 = false;
+    for (const auto& ag : p.aggs) counts32 = counts32 || (w32 && !any_multi && (ag.fn == AggFn::Count || ag.fn == AggFn::Avg));
+    meta << "rowmax " << (counts32 ? or_rows : 0ULL) << "\n";
     meta << "kernel " << kname << " scan 0 " << CTA << " " << WT << " " << smem_total << " " << tu.ctas_per_sm << "\n";
     if (grouped && !smem_groups && !reg_groups && !lane_groups) meta << "touched " << TW << "\n";
 
@@ -3333,6 +3344,10 @@ struct SharedGen {
     if (tu.cube > 0) collect_cube();
     else cube_why = "cube path switched off";
     meta << "v 2\nshared " << MAXQ << " " << MAXQ * std::max(1, max_lits) << "\n";
+    bool counts32 = false;  // per-CTA row counts of one 32-bit word, in both paths
+    for (const Plan* sh : shapes)
+      for (const auto& ag : sh->aggs) counts32 = counts32 || ag.fn == AggFn::Count;
+    meta << "rowmax " << (counts32 ? 1 : 0) << "\n";
     for (const Dim& d : dims) {
       meta << "ht " << d.slot << " dkm_" << lower(d.name) << " " << d.len * 4 << "\n";
       if (d.attrs.size() > 1) meta << "dat " << d.slot << " " << d.len * 4 << "\n";
@@ -3394,7 +3409,7 @@ struct SharedGen {
   }
 
   // Words of one group in a query's shared-memory table (a SUM is a low and a
-  // high 32-bit word, a COUNT one word), the copies of each word (lane modulo
+  // high 32-bit word, a COUNT one word, see `rowmax`), the copies of each word (lane modulo
   // copies, so that lanes on one group hit different banks: 32 for a scalar or a
   // few groups) and the table's bytes; a table of more than 4 KB per query is not
   // kept (its rows go to the result with global atomics).

@@ -134,6 +134,10 @@ struct LaunchPlan {
   int shared_maxq = 256, shared_maxp = 4096;           // queries / parameters per shared launch
   uint64_t shared_qb_bytes = 0;                        // shared memory of row bitmaps per query of a pass
   int nparams = -1;                                    // parametric plain kernels: literal count
+  // Most times one fact row adds to a per-CTA count of one 32-bit word; 0: the
+  // program has no such count.  Programs without the line may have been
+  // generated with any number of OR-joins: bounded as four of four keys.
+  long long rowmax = 256;
   bool rows_sized = false;                             // some hash table is sized by a table's rows
   std::map<int, uint64_t> dat_words;                   // shared scans: extra payload attributes per dimension
   std::vector<std::pair<int, std::string>> fcols;      // shared scans: fact filter table columns
@@ -170,6 +174,9 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
       // 2: shared programs whose cubes without COUNT end in presence bits (1: in words).
       if (v != 1 && v != 2) { err = "unsupported launch plan version"; return false; }
       lp.version = v;
+    } else if (k == "rowmax") {
+      ls >> lp.rowmax;
+      if (lp.rowmax < 0 || lp.rowmax > 65536) { err = "rowmax out of range"; return false; }
     } else if (k == "table") {
       int s; std::string n;
       ls >> s >> n;
@@ -393,6 +400,29 @@ uint64_t mht_payload_bytes(const LaunchPlan& lp, const std::vector<long long>& r
 }
 
 }  // namespace
+
+// Fact rows of one scan launch whose CTAs count rows in 32-bit words that start
+// at 0 and go to the 64-bit result at the launch's end: as many tile rounds of
+// `grid` CTAs (cta_rows rows each) as such a word can count, an even number of
+// them, so that every launch's rows start on a validity word and on an aligned
+// column address.  A table beyond it takes several launches, each adding to the
+// result; with every SM that is some 6e11 rows, with one SM 4.3e9 (fewer with
+// OR-joins, which count a row several times).
+static uint64_t launch_rows(const LaunchPlan& lp, uint64_t grid, uint64_t cta_rows) {
+  if (lp.rowmax == 0 || grid == 0) return UINT64_MAX;
+  const uint64_t rounds = std::max<uint64_t>(2, (0xffffffffULL / ((uint64_t)lp.rowmax * cta_rows)) & ~1ULL);
+  return grid * rounds * cta_rows;
+}
+
+// The fact table's columns and validity words from row `r0` (a multiple of 64) on.
+static void skip_rows(const LaunchPlan& lp, CxArgs& a, uint64_t r0) {
+  for (const auto& col : lp.cols) {
+    if (col.table != 0) continue;
+    a.col[col.slot] += r0;
+    if (a.nul[col.slot]) a.nul[col.slot] += r0 / 64;
+  }
+  a.rows[0] -= (long long)r0;
+}
 
 // ---------------------------------------------------------------- module ---
 struct cx_module {
@@ -1449,6 +1479,13 @@ int cx_execute_params(cx_module* m, cx_exec_ctx* c, const int32_t* params, int n
     const int per_sm = std::max(1, std::min(k.ctas_per_sm, L->occupancy[ki]));
     const long long grid = std::min<long long>((tiles + warps - 1) / warps, (long long)sms * per_sm);
     scan_grid = (int)grid;
+    const long long most = (long long)std::min<uint64_t>(launch_rows(lp, (uint64_t)grid, (uint64_t)(warps * k.tile)), INT64_MAX);
+    for (long long left = rows[0]; left > most; left -= most) {
+      a.rows[0] = most;
+      if ((rc = launch(ki, (unsigned)grid))) return rc;
+      a.rows[0] = left;
+      skip_rows(lp, a, (uint64_t)most);
+    }
     if ((rc = launch(ki, (unsigned)grid))) return rc;
     ++ki;
   }
@@ -1714,6 +1751,7 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
     int qn = 0, nparams = 0;
     size_t extra_smem = 0;
     unsigned scan_grid = 0;
+    uint64_t scan_rows = 0;  // most fact rows of one scan launch
     char* hstage = nullptr;
     CUfunction scan_fn = nullptr;  // the generic scan kernel, or its build for the batch's cube layout
   };
@@ -1780,6 +1818,8 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
     const long long tiles = (rows[0] + sk.tile - 1) / sk.tile;
     const int per_sm = std::max(1, std::min(sk.ctas_per_sm, occ));
     P.scan_grid = (unsigned)std::min<long long>(tiles, (long long)sms * per_sm);
+    // (a cube scan's tile is a warp's, a mask scan's a CTA's)
+    P.scan_rows = launch_rows(lp, P.scan_grid, (uint64_t)sk.tile * (cube ? (uint64_t)std::max(1, sk.block / 32) : 1));
   }
 
   // Enqueues the whole batch on `s`: one fixed sequence per pass shape, so a
@@ -1833,7 +1873,19 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
         if (r) return r;
       }
       if (ps == 0) CX_CUDA(rec(c->ev[1]));
-      int r = launch(scan_ki, P.scan_grid, P.extra_smem, &P.args, P.scan_fn);
+      int r = CX_OK;
+      if (range_rows <= P.scan_rows) {
+        r = launch(scan_ki, P.scan_grid, P.extra_smem, &P.args, P.scan_fn);
+      } else {
+        CxArgs part = P.args;
+        for (uint64_t left = range_rows, take; left > 0 && !r; left -= take) {
+          take = std::min(left, P.scan_rows);
+          part.rows[0] = (long long)take;
+          r = launch(scan_ki, P.scan_grid, P.extra_smem, &part, P.scan_fn);
+          part.rows[0] = (long long)left;
+          skip_rows(lp, part, take);
+        }
+      }
       if (r) return r;
       if (ps == npass - 1) CX_CUDA(rec(c->ev[2]));
       for (size_t ki = scan_ki + 1; ki < lp.kernels.size(); ++ki) {
