@@ -1734,8 +1734,11 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
   if (scan_ki == lp.kernels.size()) return fail(CX_E_INVALID, "cx_shared_execute: program has no %s kernel", scan_kind);
   const KernelSpec& sk = lp.kernels[scan_ki];
   // Shared-memory group tables go into the slack the scan's own residency
-  // leaves, so they never cost a resident CTA.
-  const int by_threads = std::max(1, 2048 / std::max(sk.block, 1));
+  // leaves, so they never cost a resident CTA.  Its registers (at most 64 a
+  // thread) allow 1,024 threads an SM: by 2,048, a 1,024-thread scan asked for
+  // two CTAs an SM got half of the shared memory for the one that fits, and 23 of
+  // 64 queries of seven groups no table (20M rows: 50 ms, with all tables 1.5).
+  const int by_threads = std::max(1, 1024 / std::max(sk.block, 1));
   const size_t qb_max = (size_t)lp.shared_qb_bytes * (size_t)std::min(nq, maxq) + 16;
   const int resident = std::max(1, std::min({sk.ctas_per_sm, by_threads, (int)(233472 / (sk.smem + qb_max + 1024))}));
   const size_t smem_cap = std::min<size_t>(200 * 1024, 233472 / resident - 1024);
