@@ -3430,6 +3430,13 @@ struct SharedGen {
     return fixed < cap ? (cap - fixed) / MAXQ : 0;
   }
 
+  // Every aggregate of a scalar query valid, 64 bits at a time.
+  static void emit_scalar_valid(std::ostream& o, const std::string& validity, int naggs) {
+    for (int k = 0; k < naggs; k += 64)
+      o << "          cx::set_valid_bits((uint64_t*)" << validity << ", " << k << "ULL, "
+        << (naggs - k >= 64 ? ~0ULL : (1ULL << (naggs - k)) - 1ULL) << "ULL);\n";
+  }
+
   // Words of one group in a query's shared-memory table (a SUM is a low and a
   // high 32-bit word, a COUNT one word, see `rowmax`), the copies of each word (lane modulo
   // copies, so that lanes on one group hit different banks: 32 for a scalar or a
@@ -3812,7 +3819,7 @@ struct SharedGen {
         else o << "          atomicAdd(&r_[" << k << "], x" << k << "_);\n";
       }
       if (NG) o << "          cx::set_bit_once(&s_sq[q].touched[hash >> 5], 1u << (hash & 31));\n";
-      else o << "          cx::set_valid_bits((uint64_t*)s_sq[q].validity, 0ULL, " << (NA >= 64 ? ~0ULL : (1ULL << NA) - 1ULL) << "ULL);\n";
+      else emit_scalar_valid(o, "s_sq[q].validity", NA);
       o << "        }\n";
       o << "      }\n";
     }
@@ -3861,7 +3868,7 @@ struct SharedGen {
       for (int k = 0; k < NA; ++k)
         o << "          if (v" << k << "_) atomicAdd(&Q.result[(unsigned long long)g * " << TS << "ULL + " << NG + k << "], v" << k << "_);\n";
       if (NG) o << "          cx::set_bit_once(&Q.touched[g >> 5], 1u << (g & 31));\n";
-      else o << "          cx::set_valid_bits((uint64_t*)Q.validity, 0ULL, " << (NA >= 64 ? ~0ULL : (1ULL << NA) - 1ULL) << "ULL);\n";
+      else emit_scalar_valid(o, "Q.validity", NA);
       o << "        }\n        break;\n";
     }
     o << "      default: break;\n";
