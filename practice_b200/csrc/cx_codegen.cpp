@@ -3440,12 +3440,20 @@ struct SharedGen {
   // Words of one group in a query's shared-memory table (a SUM is a low and a
   // high 32-bit word, a COUNT one word, see `rowmax`), the copies of each word (lane modulo
   // copies, so that lanes on one group hit different banks: 32 for a scalar or a
-  // few groups) and the table's bytes; a table of more than 4 KB per query is not
-  // kept (its rows go to the result with global atomics).  Copies take no more
+  // few groups) and the table's bytes.  Copies take no more
   // than a query's share of a full pass, so that no query is left without its
   // table for other queries' copies: 64 queries of ten groups (SUM and COUNT)
   // with 3,840 bytes each spent 46 ms on 20M rows, of 1,920 bytes 1.6 ms.
-  struct QTab { int words = 0, rep = 1; unsigned long long u64 = 0, bits = 0; bool counts = false; };
+  //
+  // A wider domain gets a table of `slots` groups, whichever come first: a tag
+  // (group + 1) and the words each.  Rows of the groups in it are added there, the
+  // others to the result.  Few live groups of a wide domain (skewed keys, a
+  // selective join) otherwise queue at a few addresses of the result: 20M rows in
+  // 11 of 5,000 groups, 1 / 8 / 32 queries 3.9 / 9.0 / 11.2 -> 0.12 / 0.33 / 1.04 ms
+  // (merging equal groups across a warp instead: 2.1 / 2.5 / 6.6).  Where nearly
+  // every row is a group of its own the tag test costs: 16 queries of 62,500
+  // groups 0.354 -> 0.399.  16 to 256 slots measure alike; 128 take 1.5 KB.
+  struct QTab { int words = 0, rep = 1, slots = 0; unsigned long long u64 = 0, bits = 0; bool counts = false; };
   QTab qtab_of(const Plan& p) const {
     QTab t;
     Emitter e(p, tu);
@@ -3455,7 +3463,14 @@ struct SharedGen {
       t.counts = t.counts || ag.fn == AggFn::Count;
     }
     const unsigned long long one = G * t.words * 4;
-    if (one > 4096) return t;
+    if (one > 4096) {
+      const unsigned long long room = std::min<unsigned long long>(4096, qtab_budget()), slot = (t.words + 1) * 4ULL;
+      if (p.groups.empty() || 16 * slot + 8 > room) return t;
+      t.slots = 16;
+      while (2 * t.slots * slot + 8 <= room && t.slots < 128) t.slots *= 2;
+      t.u64 = (t.slots * slot + 7) / 8;
+      return t;
+    }
     t.bits = t.counts ? 0 : (G + 31) / 32;
     while (t.rep < 32 && one * t.rep * 2 + t.bits * 4 + 8 <= qtab_budget() && one * t.rep * 2 <= 4096) t.rep *= 2;
     t.u64 = (one * t.rep + 7) / 8;
@@ -3790,9 +3805,22 @@ struct SharedGen {
       }
       if (qt.u64) {
         o << "          const int2 qt_ = s_qt[q];\n";
-        o << "          if (qt_.x >= 0) {\n";
-        o << "            unsigned* w_ = s_tab + qt_.x + (unsigned)hash * " << qt.words * qt.rep << "u"
-          << (qt.rep > 1 ? " + (lane & " + std::to_string(qt.rep - 1) + ")" : std::string()) << ";\n";
+        if (qt.slots) {
+          int sh = 32;
+          while ((1 << (32 - sh)) < qt.slots) --sh;
+          o << "          unsigned at_ = 0u, own_ = 0u;\n";
+          o << "          if (qt_.x >= 0) {\n";
+          o << "            at_ = ((unsigned)hash * 2654435769u) >> " << sh << ";\n";
+          o << "            own_ = *(volatile unsigned*)(s_tab + qt_.x + at_);\n";
+          o << "            if (own_ == 0u) { own_ = atomicCAS(s_tab + qt_.x + at_, 0u, (unsigned)hash + 1u); if (own_ == 0u) own_ = (unsigned)hash + 1u; }\n";
+          o << "          }\n";
+          o << "          if (own_ == (unsigned)hash + 1u) {\n";
+          o << "            unsigned* w_ = s_tab + qt_.x + " << qt.slots << "u + at_ * " << qt.words << "u;\n";
+        } else {
+          o << "          if (qt_.x >= 0) {\n";
+          o << "            unsigned* w_ = s_tab + qt_.x + (unsigned)hash * " << qt.words * qt.rep << "u"
+            << (qt.rep > 1 ? " + (lane & " + std::to_string(qt.rep - 1) + ")" : std::string()) << ";\n";
+        }
         int w = 0;
         bool first = true;
         for (int k = 0; k < NA; ++k) {
@@ -3805,7 +3833,7 @@ struct SharedGen {
           o << "              const unsigned xh_ = (unsigned)(" << x << " >> 32) + (old_ + xl_ < xl_ ? 1u : 0u);\n";
           o << "              if (xh_) atomicAdd(&w_[" << (w + 1) * qt.rep << "], xh_);\n";
           // The first row of a copy finds its low word 0.
-          if (first && !qt.counts) o << "              if (old_ == 0u) cx::set_bit_once(&s_bits[qt_.y + (hash >> 5)], 1u << (hash & 31));\n";
+          if (first && !qt.counts && !qt.slots) o << "              if (old_ == 0u) cx::set_bit_once(&s_bits[qt_.y + (hash >> 5)], 1u << (hash & 31));\n";
           o << "            }\n";
           first = false;
           w += 2;
@@ -3845,10 +3873,15 @@ struct SharedGen {
       const int TS = p.storage_ts(), NA = (int)p.aggs.size(), NG = (int)p.groups.size();
       const bool by_warp = qt.rep == 32;
       o << "      case " << s << ":\n";
-      if (by_warp) o << "        for (int g = (warp + q) % " << NW << "; g < " << G << "; g += " << NW << ") {\n";
+      if (qt.slots) {
+        o << "        for (int at_ = threadIdx.x; at_ < " << qt.slots << "; at_ += " << CTA << ") {\n";
+        o << "          const unsigned g = s_tab[s_qt[q].x + at_] - 1u;\n";
+        o << "          if (g == ~0u) continue;\n";
+      } else if (by_warp) o << "        for (int g = (warp + q) % " << NW << "; g < " << G << "; g += " << NW << ") {\n";
       else o << "        for (int g = threadIdx.x; g < " << G << "; g += " << CTA << ") {\n";
-      if (!qt.counts) o << "          if (!((qb_[g >> 5] >> (g & 31)) & 1u)) continue;\n";
-      o << "          const unsigned* w_ = s_tab + s_qt[q].x + (unsigned)g * " << qt.words * qt.rep << "u;\n";
+      if (!qt.counts && !qt.slots) o << "          if (!((qb_[g >> 5] >> (g & 31)) & 1u)) continue;\n";
+      if (qt.slots) o << "          const unsigned* w_ = s_tab + s_qt[q].x + " << qt.slots << "u + (unsigned)at_ * " << qt.words << "u;\n";
+      else o << "          const unsigned* w_ = s_tab + s_qt[q].x + (unsigned)g * " << qt.words * qt.rep << "u;\n";
       int w = 0;
       std::string any;
       for (int k = 0; k < NA; ++k) {
