@@ -3660,6 +3660,13 @@ struct SharedGen {
     for (const auto& c : fact_cols) o << "    int c_" << c << "[IPT];\n";
     o << "    if (nt == TROWS && vec_ok && m_cols == " << every << "ULL) {\n";
     for (const auto& c : fact_cols) o << "      WarpLoadTileV<IPT>(d_" << c << " + base, lane, c_" << c << ");\n";
+    // (a pass with some of the program's shapes reads some of its columns)
+    o << "    } else if (nt == TROWS && vec_ok) {\n";
+    for (size_t k = 0; k < NSC; ++k) {
+      const std::string& c = fact_cols[k];
+      o << "      if ((m_cols >> " << k << ") & 1ULL) WarpLoadTileV<IPT>(d_" << c << " + base, lane, c_" << c << ");\n";
+      o << "      else {\n        #pragma unroll\n        for (int i = 0; i < IPT; ++i) c_" << c << "[i] = 0;\n      }\n";
+    }
     o << "    } else {\n";
     o << "      #pragma unroll\n";
     o << "      for (int i = 0; i < IPT; ++i) {\n";
