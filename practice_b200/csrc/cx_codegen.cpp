@@ -621,13 +621,14 @@ struct Emitter {
       used += bytes;
     }
   }
+  static long long bitmap_words(const Join& j) { return (j.len + 31) / 32; }
   // Joins whose membership bitmap the scan keeps in shared memory: in join
   // order, while the bitmaps fit the budget.
   void choose_bitmaps() {
     unsigned long long used = 0;
     for (const auto& s : p.steps) {
       if (s.kind != Step::JoinStep || s.join.expands() || !exact_window_ok(s.join) || ptable.count(s.join.dim)) continue;
-      const unsigned long long bytes = (((unsigned long long)(s.join.len + 31) / 32) * 4 + 15) & ~15ULL;
+      const unsigned long long bytes = ((unsigned long long)bitmap_words(s.join) * 4 + 15) & ~15ULL;
       if (used + bytes > (unsigned long long)std::max(0, tu.bitmap_budget)) continue;
       bitmaps.insert(s.join.dim);
       used += bytes;
@@ -821,7 +822,7 @@ struct Emitter {
         if (s.kind != Step::JoinStep) continue;
         const bool table = ptable.count(s.join.dim) > 0;
         if (!table && !bitmaps.count(s.join.dim)) continue;
-        const unsigned long long words = (unsigned long long)(table ? (s.join.len + 3) / 4 : s.join.len / 32 + 1);
+        const unsigned long long words = (unsigned long long)(table ? (s.join.len + 3) / 4 : bitmap_words(s.join));
         off = (off + 15) & ~15ULL;
         sbms.push_back({s.join.dim, s.join.fks[0], ht_slot.at(s.join.dim), s.join.len, s.join.keymin, words, off,
                         !s.join.payload.empty(), table, s.join.prange_min});
@@ -2290,7 +2291,7 @@ struct Emitter {
       if (!s.join.payload.empty() && payload_valid.count(s.join.payload))
         meta << "htv " << h << " " << (s.join.len + 31) / 32 << "\n";
       if (ptable.count(s.join.dim)) meta << "bm " << h << " " << (s.join.len + 3) / 4 << "\n";
-      else if (bitmaps.count(s.join.dim)) meta << "bm " << h << " " << s.join.len / 32 + 1 << "\n";  // (bit len is 0)
+      else if (bitmaps.count(s.join.dim)) meta << "bm " << h << " " << bitmap_words(s.join) << "\n";
       ++h;
     }
     if (h > CX_MAX_HTS_) throw PlanError("too many joins");
