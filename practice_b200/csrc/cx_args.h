@@ -100,4 +100,5 @@ struct CxArgs {
   long long zero_bytes;
   int zero_parts;                              // shared passes: blocks per query of the zeroing and key kernels
   int zero_err;                                // 1: the zeroing kernel clears the error word too
+  int build_cap;                               // most blocks of one table's part of a build kernel
 };

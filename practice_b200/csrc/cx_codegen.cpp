@@ -396,16 +396,16 @@ struct Emitter {
     return "__device__ __forceinline__ void " + name + "(const CxArgs& a, long long cx_block, long long cx_blocks) {\n";
   }
   // One kernel over the parts of several dimensions, one launch instead of one
-  // per dimension: table `t` gets a block per 512 rows, at most kBuildCap.
-  static constexpr int kBuildCap = 148 * 16;
+  // per dimension: table `t` gets a block per 512 rows, at most `build_cap` (16
+  // per SM of the context's count).
   void emit_part_kernel(const std::string& kname, const std::vector<std::pair<std::string, int>>& parts) {
-    meta << "kernel " << kname << " builds 0 128 512 " << kBuildCap << " " << parts.size();
+    meta << "kernel " << kname << " builds 0 128 512 0 " << parts.size();
     for (const auto& pt : parts) meta << " " << pt.second;
     meta << "\n";
     src << "extern \"C\" __global__ void __launch_bounds__(128) " << kname << "(const CxArgs a) {\n";
     src << "  long long cx_b = blockIdx.x;\n";
     for (const auto& pt : parts) {
-      src << "  { const long long cx_n = cx::build_blocks(a.rows[" << pt.second << "], 512, " << kBuildCap << ");\n";
+      src << "  { const long long cx_n = cx::build_blocks(a.rows[" << pt.second << "], 512, a.build_cap);\n";
       src << "    if (cx_b < cx_n) { " << pt.first << "(a, cx_b, cx_n); return; }\n";
       src << "    cx_b -= cx_n; }\n";
     }
@@ -2624,13 +2624,13 @@ struct SharedGen {
   // rows; one after another, four of these kernels took 20 us of a small batch).
   void emit_index_kernel(const char* kname, const char* kind, const std::vector<std::pair<std::string, int>>& parts) {
     if (parts.empty()) return;
-    meta << "kernel " << kname << " " << kind << " 0 256 256 " << 148 * 16 << " " << parts.size();
+    meta << "kernel " << kname << " " << kind << " 0 256 256 0 " << parts.size();
     for (const auto& pt : parts) meta << " " << pt.second;
     meta << "\n";
     src << "extern \"C\" __global__ void __launch_bounds__(256) " << kname << "(const CxArgs a) {\n";
     src << "  long long cx_b = blockIdx.x;\n";
     for (const auto& pt : parts) {
-      src << "  { const long long cx_n = cx::build_blocks(a.rows[" << pt.second << "], 256, " << 148 * 16 << ");\n";
+      src << "  { const long long cx_n = cx::build_blocks(a.rows[" << pt.second << "], 256, a.build_cap);\n";
       src << "    if (cx_b < cx_n) { " << pt.first << "(a, cx_b, cx_n); return; }\n";
       src << "    cx_b -= cx_n; }\n";
     }

@@ -105,7 +105,7 @@ struct KernelSpec {
   std::string name, kind;
   int table = 0, block = 128, tile = 512, ctas_per_sm = 1;
   size_t smem = 0;
-  int cap = 0;                // "builds": most blocks of one table
+  int cap = 0;                // "builds": most blocks of one table (0: CxArgs.build_cap)
   std::vector<int> parts;     // "builds": tables, each with its own range of blocks
 };
 
@@ -326,7 +326,7 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
     }
   for (const auto& k : lp.kernels) {
     if (k.kind != "builds" && k.kind != "cubebuilds") continue;
-    bool ok = k.tile > 0 && k.block > 0 && k.block <= 1024 && k.cap > 0 && !k.parts.empty();
+    bool ok = k.tile > 0 && k.block > 0 && k.block <= 1024 && k.cap >= 0 && !k.parts.empty();
     for (int t : k.parts) ok = ok && t >= 0 && t < (int)lp.tables.size();
     if (!ok) {
       err = "kernel line " + k.name + " names a table outside the plan or a bad shape";
@@ -422,6 +422,11 @@ static void skip_rows(const LaunchPlan& lp, CxArgs& a, uint64_t r0) {
     if (a.nul[col.slot]) a.nul[col.slot] += r0 / 64;
   }
   a.rows[0] -= (long long)r0;
+}
+
+// Blocks of one table's part of a build kernel, by the kernel's own rule.
+static unsigned part_blocks(const KernelSpec& k, long long rows, int build_cap) {
+  return (unsigned)std::min<long long>((rows + k.tile - 1) / k.tile, k.cap ? k.cap : build_cap);
 }
 
 // ---------------------------------------------------------------- module ---
@@ -1418,6 +1423,7 @@ int cx_execute_params(cx_module* m, cx_exec_ctx* c, const int32_t* params, int n
 
   int sms = c->sm_override;
   if (sms <= 0) CX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  a.build_cap = (int)std::min<long long>((long long)sms * 16, INT32_MAX);
 
   Driver& d = driver();
   int launches = 0, scan_grid = 0;
@@ -1456,7 +1462,7 @@ int cx_execute_params(cx_module* m, cx_exec_ctx* c, const int32_t* params, int n
       const long long tiles = (rows[k.table] + k.tile - 1) / k.tile;
       grid = (unsigned)std::min<long long>(tiles, (long long)sms * 16);
     } else if (k.kind == "builds") {
-      for (int t : k.parts) grid += (unsigned)std::min<long long>((rows[t] + k.tile - 1) / k.tile, k.cap);
+      for (int t : k.parts) grid += part_blocks(k, rows[t], a.build_cap);
     } else if (k.kind == "tiles") {
       // One CTA per tile of the table (a translated nd_range kernel).
       grid = (unsigned)((rows[k.table] + k.tile - 1) / k.tile);
@@ -1745,6 +1751,7 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
 
   int sms = c->sm_override;
   if (sms <= 0) CX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  a.build_cap = (int)std::min<long long>((long long)sms * 16, INT32_MAX);
   Driver& d = driver();
 
   // Plan every pass on the host: descriptors and parameters into the pinned
@@ -1868,7 +1875,7 @@ int cx_shared_execute_rows(cx_module* m, cx_exec_ctx* c, const cx_shared_query* 
                             std::min<uint64_t>(((uint64_t)P.args.zero_bytes / 16 + k.block - 1) / k.block, (uint64_t)sms * 8));
         else if (k.kind == "zero") grid = (unsigned)P.qn;
         else if (k.kind == (cube ? "cubebuilds" : "builds"))
-          for (int t : k.parts) grid += (unsigned)std::min<long long>((rows[t] + k.tile - 1) / k.tile, k.cap);
+          for (int t : k.parts) grid += part_blocks(k, rows[t], a.build_cap);
         else if (k.kind == (cube ? "cubeidx" : "build"))
           grid = (unsigned)std::min<long long>((rows[k.table] + k.tile - 1) / k.tile, (long long)sms * 16);
         else continue;
