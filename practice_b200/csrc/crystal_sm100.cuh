@@ -1260,5 +1260,56 @@ CX_DEVICE void warp_group_add(bool active, int group, unsigned long long v, Appl
   if (lane == leader) apply(group, sum);
 }
 
+// The next two serve shared programs whose text an earlier generator wrote; it is
+// accepted by cx_compile as before.
+
+// 32x32 bit-matrix transpose across a warp: lane r passes row r; lane c gets
+// column c (bit r of the result = bit c of lane r's row).  Five exchange
+// steps swap the off-diagonal blocks of 16, 8, 4, 2 and 1 bits (the
+// recursive block transpose of Hacker's Delight 7-3, one row per lane).
+// Every lane of the warp must call it.
+CX_DEVICE unsigned warp_transpose32(unsigned x, int lane) {
+  const unsigned masks[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    const int j = 16 >> s;
+    const unsigned m = masks[s];
+    const unsigned y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
+  }
+  return x;
+}
+
+// Warp reduce-scatter of P (a power of two <= 32) per-lane u64 values.  Each
+// exchange step halves the values a lane carries: the lane keeps the half its
+// lane bit selects and adds the partner's copy of it; once one value is left
+// the remaining steps are a plain butterfly.  Returns the value index whose
+// warp total the lane then holds in v[0]; lanes with (lane & (32 / P - 1)) == 0
+// hold each index exactly once.  Every lane of the warp must call it.
+template <int P>
+CX_DEVICE int warp_reduce_scatter_u64(unsigned long long (&v)[P], int lane) {
+  static_assert(P >= 1 && P <= 32 && (P & (P - 1)) == 0, "P must be a power of two <= 32");
+  int idx = 0;
+  int cnt = P;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (cnt > 1) {
+      const int h = cnt / 2;
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int k = 0; k < h; ++k) {
+        const unsigned long long send = up ? v[k] : v[k + h];
+        const unsigned long long keep = up ? v[k + h] : v[k];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+      if (up) idx += h;
+      cnt = h;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return idx;
+}
+
 }  // namespace cx
 

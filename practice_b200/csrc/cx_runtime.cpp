@@ -288,6 +288,9 @@ bool parse_launch_plan(const std::string& src, LaunchPlan& lp, std::string& err)
       lp.finalize = true;
       ls >> lp.fin_groups >> lp.fin_vts;
     } else if (k == "kernel") {
+      // ("build", "cubeidx", "zero", "queries", plans without "prep" or "zeroall",
+      // caps above 0 and the `sqb` line come from earlier generators; programs
+      // that kept such a text still load and run.)
       KernelSpec ks;
       ls >> ks.name >> ks.kind >> ks.table >> ks.block;
       if (ks.kind == "build" || ks.kind == "cubeidx" || ks.kind == "tiles" || ks.kind == "tilescan") ls >> ks.tile;
