@@ -249,15 +249,12 @@ PLAIN_CANDIDATES = [dict(block_threads=bt, items_per_thread=ipt, stages=st, ctas
                         (1024, 2, 0, 49152, 1, 0, 1, 0), (1024, 4, 0, 49152, 1, 0, 2, 0),
                         (1024, 2, 0, 49152, 1, 0, 2, 0), (1024, 4, 0, 49152, 3, 0, 0, 98304),
                         (1024, 8, 0, 49152, 1, 0, 2, 0))]
-# Per-query mask path (cube = 0) launch shapes, then the aggregate-cube path at
+# Per-query mask path (cube = 0) by block size, then the aggregate-cube path at
 # 1, 2 and 4 rows per lane (the runtime falls back to the mask path when the
-# batch's attribute ranges do not allow cubes).
-SHARED_CANDIDATES = [dict(block_threads=bt, items_per_thread=ipt, stages=st, ctas_per_sm=2, producer_warps=pw,
-                          group_merge=gm, cube=0)
-                     for bt, ipt, st, pw, gm in ((1024, 1, 3, 11, 0), (1024, 1, 3, 11, 3), (1024, 1, 3, 14, 0),
-                                                 (1024, 1, 3, 14, 3), (512, 2, 2, 5, 0), (512, 2, 2, 7, 3))]
-SHARED_CANDIDATES += [dict(block_threads=1024, items_per_thread=1, stages=3, ctas_per_sm=2, producer_warps=11,
-                           group_merge=3, cube=c) for c in (1, 2, 4)]
+# batch's attribute ranges do not allow cubes).  Other knobs do not change a
+# shared scan's kernels.
+SHARED_CANDIDATES = [dict(block_threads=1024, items_per_thread=1, stages=3, ctas_per_sm=2, cube=c) for c in (0, 1, 2, 4)]
+SHARED_CANDIDATES.insert(1, dict(block_threads=512, items_per_thread=2, stages=2, ctas_per_sm=2, cube=0))
 
 
 def bound_ctx(db, module, res, val):
