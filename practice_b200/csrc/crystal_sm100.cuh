@@ -994,6 +994,7 @@ CX_DEVICE void mbar_init(unsigned long long* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
 CX_DEVICE void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+// (this fence and mbar_arrive serve program texts of an earlier generator)
 CX_DEVICE void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 CX_DEVICE void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {

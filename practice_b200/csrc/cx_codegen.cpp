@@ -2346,7 +2346,7 @@ std::string generate_cuda_impl(const Plan& plan, const Tuning& tuning) {
 // into one 64-bit query mask per fact row (bit q set: the row passes query q),
 // in the manner of the CJOIN shared star-join operator (Candea, Polyzotis,
 // Vingralek, VLDB 2009):
-//  * index_<dim> kernels store, at the PHT slot HASH(key, len, key_min) of each
+//  * index_tables stores, at the PHT slot HASH(key, len, key_min) of each
 //    dimension row, {key, mask_lo, mask_hi, attr0} and up to three more payload
 //    attributes.  Mask bit q is set when query q does not join the dimension or
 //    the row passes the query's dimension filter -- the condition under which
@@ -2357,9 +2357,10 @@ std::string generate_cuda_impl(const Plan& plan, const Tuning& tuning) {
 //    FW values of the column, starting at the column minimum the host
 //    registered; values outside the window, and every other filter, are
 //    evaluated per query for the rows still in the mask.
-//  * warps then take (query, row slice) units and aggregate the rows whose bit
-//    is set, four rows per lane, with partial aggregates in registers, a
-//    per-query shared-memory table or global atomics.
+//  * a lane keeps the masks of two rows in registers, takes each shape's group and
+//    aggregate values once per row, and adds them for every set bit to that
+//    query's table in shared memory, or to its result where the table does not
+//    hold the group.
 
 void lits_of(const Expr* e, std::vector<const Expr*>& out) {
   if (!e) return;
@@ -2583,10 +2584,7 @@ struct SharedGen {
     return out.empty() ? "true" : out;
   }
 
-  // Per pass: zeroes every query's result words, validity words and touched
-  // bits (one block per query), so a pass has the same launches whatever its
-  // queries' buffers are.
-  // What a pass starts from, in one launch: each query's result and validity
+  // What a pass starts from, in one launch whatever its queries' buffers are: each query's result and validity
   // words (zero_parts blocks a query), then the scratch -- dimension entries,
   // touched bits, aggregate cubes -- and before the first pass the error word.
   // One block per query took 10 us for 28,000 words and 30 ms for a 330 MB

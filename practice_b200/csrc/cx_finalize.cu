@@ -421,7 +421,7 @@ __device__ __forceinline__ unsigned rows_before(const unsigned long long* __rest
 // 64 runs x 10 steps at 80 dependent loads per thread.  The last pass writes
 // the result columns (rank < limit) straight from the group table; an earlier
 // one writes the merged run.  Measured, cx_finalize as a whole on a 62,500-group
-// result ordered by two columns: 75 us; 1,300 us as a network of 136 global
+// result ordered by two columns: 61 us; 1,300 us as a network of 136 global
 // compare-exchange launches with its scratch from the default pool.
 __global__ void __launch_bounds__(256) fin_merge_runs(const unsigned long long* __restrict__ src,
                                                       const unsigned long long* __restrict__ val, const FinDesc d,
