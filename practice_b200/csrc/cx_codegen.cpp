@@ -3062,8 +3062,9 @@ struct SharedGen {
     // lane interleave: with a branch per row and shape the kernel spent 2.7 of
     // 11.6 cycles per instruction on fixed latencies and 1.1 on branches.
     // Measured (32 mixed queries): 60M rows 0.545 -> 0.463 ms, 600M rows 5.04 ->
-    // 4.25 ms; what is left is bound by the L1 pipe (66 % of its wavefronts, two
-    // thirds of them the random customer and part gathers) and issue (73 %).
+    // 4.25 ms; what is left is bound by issue (70 % of the cycles, 180M warp
+    // instructions for 30M rows) and the L1 pipe (68 % of its wavefronts; the
+    // customer and part gathers touch 17 sectors a request).
     std::vector<std::vector<std::string>> xs(shapes.size());
     for (size_t s = 0; s < shapes.size(); ++s) {
       const Plan& p = *shapes[s];
@@ -3437,18 +3438,18 @@ struct SharedGen {
   }
 
   // Words of one group in a query's shared-memory table (a SUM is a low and a
-  // high 32-bit word, a COUNT one word, see `rowmax`), the copies of each word (lane modulo
-  // copies, so that lanes on one group hit different banks: 32 for a scalar or a
-  // few groups) and the table's bytes.  Copies take no more
-  // than a query's share of a full pass, so that no query is left without its
-  // table for other queries' copies: 64 queries of ten groups (SUM and COUNT)
-  // with 3,840 bytes each spent 46 ms on 20M rows, of 1,920 bytes 1.6 ms.
+  // high 32-bit word, a COUNT one word, see `rowmax`), the copies of each word
+  // (lane modulo copies, so that lanes on one group hit different banks: 32 for a
+  // scalar or a few groups) and the table's bytes.  Copies take no more than a
+  // query's share of a full pass, so that no query is left without its table for
+  // other queries' copies: 64 queries of ten groups (SUM and COUNT) with 3,840
+  // bytes each spent 46 ms on 20M rows, of 1,920 bytes 1.6 ms.
   //
   // A wider domain gets a table of `slots` groups, whichever come first: a tag
-  // (group + 1) and the words each.  Rows of the groups in it are added there, the
-  // others to the result.  Few live groups of a wide domain (skewed keys, a
+  // (group + 1) and the words each.  Rows of the groups in it are added there,
+  // those of the others to the result.  Few live groups of a wide domain (skewed keys, a
   // selective join) otherwise queue at a few addresses of the result: 20M rows in
-  // 11 of 5,000 groups, 1 / 8 / 32 queries 3.9 / 9.0 / 11.2 -> 0.12 / 0.33 / 1.04 ms
+  // 11 of 5,000 groups, 1 / 8 / 32 queries 3.9 / 9.0 / 11.2 -> 0.12 / 0.33 / 0.98 ms
   // (merging equal groups across a warp instead: 2.1 / 2.5 / 6.6).  Where nearly
   // every row is a group of its own the tag test costs: 16 queries of 62,500
   // groups 0.354 -> 0.399.  16 to 256 slots measure alike; 128 take 1.5 KB.
@@ -3510,8 +3511,9 @@ struct SharedGen {
   // bitmaps per query, transposed, walked bit by bit) a 32-query batch took
   // 798 warp instructions per 32 rows, most of them for the hand-over.
   // Measured at 60M rows, scan: 8 / 16 / 32 / 64 mixed queries 1.77 / 1.83 /
-  // 2.05 / 3.27 -> 1.00 / 1.19 / 1.47 / 2.23 ms; bound by the L1 pipe (a 16-byte
-  // gather per joined dimension and row, each lane its own line) and issue.
+  // 2.05 / 3.27 -> 1.02 / 1.21 / 1.50 / 2.27 ms; bound by issue (71 % of the
+  // cycles) and the waits on shared memory and on the gathers, 16 bytes per joined
+  // dimension and row, each lane its own line (16 sectors a request).
   void emit_scan() {
     const int CTA = tu.block_threads;
     if (CTA % 32 || CTA < 64 || CTA > 1024 || tu.items_per_thread < 1 || tu.items_per_thread > 16) throw PlanError("bad block shape");
@@ -3814,14 +3816,15 @@ struct SharedGen {
         if (qt.slots) {
           int sh = 32;
           while ((1 << (32 - sh)) < qt.slots) --sh;
-          o << "          unsigned at_ = 0u, own_ = 0u;\n";
+          o << "          unsigned* w_ = s_tab;\n";
+          o << "          unsigned own_ = 0u;\n";
           o << "          if (qt_.x >= 0) {\n";
-          o << "            at_ = ((unsigned)hash * 2654435769u) >> " << sh << ";\n";
-          o << "            own_ = *(volatile unsigned*)(s_tab + qt_.x + at_);\n";
-          o << "            if (own_ == 0u) { own_ = atomicCAS(s_tab + qt_.x + at_, 0u, (unsigned)hash + 1u); if (own_ == 0u) own_ = (unsigned)hash + 1u; }\n";
+          o << "            w_ += qt_.x + (((unsigned)hash * 2654435769u) >> " << sh << ") * " << qt.words + 1 << "u;\n";
+          o << "            own_ = *(volatile unsigned*)w_;\n";
+          o << "            if (own_ == 0u) { own_ = atomicCAS(w_, 0u, (unsigned)hash + 1u); if (own_ == 0u) own_ = (unsigned)hash + 1u; }\n";
           o << "          }\n";
           o << "          if (own_ == (unsigned)hash + 1u) {\n";
-          o << "            unsigned* w_ = s_tab + qt_.x + " << qt.slots << "u + at_ * " << qt.words << "u;\n";
+          o << "            ++w_;\n";
         } else {
           o << "          if (qt_.x >= 0) {\n";
           o << "            unsigned* w_ = s_tab + qt_.x + (unsigned)hash * " << qt.words * qt.rep << "u"
@@ -3881,12 +3884,12 @@ struct SharedGen {
       o << "      case " << s << ":\n";
       if (qt.slots) {
         o << "        for (int at_ = threadIdx.x; at_ < " << qt.slots << "; at_ += " << CTA << ") {\n";
-        o << "          const unsigned g = s_tab[s_qt[q].x + at_] - 1u;\n";
+        o << "          const unsigned g = s_tab[s_qt[q].x + at_ * " << qt.words + 1 << "] - 1u;\n";
         o << "          if (g == ~0u) continue;\n";
       } else if (by_warp) o << "        for (int g = (warp + q) % " << NW << "; g < " << G << "; g += " << NW << ") {\n";
       else o << "        for (int g = threadIdx.x; g < " << G << "; g += " << CTA << ") {\n";
       if (!qt.counts && !qt.slots) o << "          if (!((qb_[g >> 5] >> (g & 31)) & 1u)) continue;\n";
-      if (qt.slots) o << "          const unsigned* w_ = s_tab + s_qt[q].x + " << qt.slots << "u + (unsigned)at_ * " << qt.words << "u;\n";
+      if (qt.slots) o << "          const unsigned* w_ = s_tab + s_qt[q].x + (unsigned)at_ * " << qt.words + 1 << "u + 1u;\n";
       else o << "          const unsigned* w_ = s_tab + s_qt[q].x + (unsigned)g * " << qt.words * qt.rep << "u;\n";
       int w = 0;
       std::string any;
