@@ -96,7 +96,7 @@ def tour(args) -> None:
     """Runs every kernel of the library once or twice on a generated table:
     the plain fused scan (Q1.1-, Q3.1- and nullable Q3.1-shaped queries, a
     parametric one, AVG finalisation, an OR-join and two multi-value hash
-    joins with their five build kernels), a shared-scan batch, result
+    joins with their build kernels), a shared-scan batch, result
     finalisation on the device and sparse compaction (both entry points)."""
     import numpy as np
 
